@@ -27,7 +27,7 @@ UNITS = {
     "serve.cu": [],
     "damping.cu": [],
 }
-HEADERS = ["internal.h", "mhd_body.cuh", "random_forcing.cuh", "filter_body.cuh",
+HEADERS = ["internal.h", "mhd_body.cuh", "quiet_body.cuh", "random_forcing.cuh", "filter_body.cuh",
            "tmem_window.cuh", "tma_util.cuh"]
 # host C units (gcc): the .trol reader
 HOST_UNITS = {"sparc_trol.c": ["-O2", "-std=c99", "-Wall", "-fPIC"]}

@@ -30,7 +30,7 @@ struct FaceT {
   R *vars;              // RK state (zpmlvars...), cnt*P
   R *scr;               // stage right-hand side (scrzpml...), cnt*P
   const R *pa, *pb, *pk;
-  const R *pki;         // 1/kappa (precision form)
+  const R *pki;         // 1/kappa
 };
 using FaceDev = FaceT<double>;
 
@@ -167,6 +167,10 @@ enum {
   FB_BOZ, FB_CBX, FB_CBY, FB_CBZ, FB_GRX, FB_GRY, FB_GPX, FB_GPY, FB_RED, FB_COUNT
 };
 
+// largest z chunk of a quiet stage block: its layer profiles sit in shared
+// memory, and longer chunks let the blocks of neighbouring tiles drift apart
+constexpr int QUIET_ZMAX = 32;
+
 struct Handle {
   sparc_params P{};
   int device = 0;
@@ -265,8 +269,8 @@ struct Handle {
   unsigned *d_wctr64 = nullptr;
   int partials_blocks = 0;  // blocks the partials hold: any z chunk >= 11
 
-  // stage launch geometry (quiet tiles tx x ty; MHD tiles 32 x 8)
-  int tx = 32, ty = 8, zchunk = 32;
+  // layers per z chunk of the stage work items (tiles of 32 x 8 columns)
+  int zchunk = 32;
 
   // precision form (SPARC_FP32): FP32 state in fbuf (roles ra/rf1/rf2 as
   // for buf), the compensated-sum carry of the state, depth scales

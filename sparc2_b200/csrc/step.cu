@@ -19,6 +19,7 @@
 
 #include "filter_body.cuh"
 #include "mhd_body.cuh"
+#include "quiet_body.cuh"
 #include "random_forcing.cuh"
 
 namespace sparc {
@@ -44,399 +45,108 @@ int step_constants() {
 }
 
 
-// CPML correction of one derivative (RHS.f90:50-93, 424-546):
-// RHSpsi = a*d + b*psi ; d = d/kappa + psi.  LAST applies the final RK
-// update of the auxiliary field in place (step.f90:59-61).
-template <int MODE>
-__device__ __forceinline__ void cpml(const FaceDev &F, long long f, int layer,
-                                     int slot, double beta, double dt,
-                                     double &d) {
-  const long long pf = F.uniform ? (long long)layer : f;
-  const double pa = __ldg(F.pa + pf), pb = __ldg(F.pb + pf),
-               pk = __ldg(F.pk + pf);
-  const long long o = (long long)slot * F.cnt + f;
-  const double v = F.vars[o];
-  double psi = v;
-  if (MODE != FIRST) psi = v + beta * F.scr[o];
-  const double rhs = pa * d + pb * psi;
-  d = d / pk + psi;
-  if (MODE == LAST) F.vars[o] = v + dt * rhs;
-  else F.scr[o] = rhs;
-}
-
-// Forcing of driver.f90:137-153 at point (i, j, k) of iteration `it`.
-__device__ __forceinline__ double forcing_at(const SimDev &S, long long it,
-                                             double T, int i, int j, int k) {
-  const ForcingDev &F = S.frc;
-  if (F.kind == SPARC_SRC_PULSE)
-    return T * __ldg(F.fz + k) * (__ldg(F.fy + j) * __ldg(F.fx + i));
-  if (F.kind == SPARC_SRC_PSR && k >= F.klo && k < F.khi)
-    return F.psr[((long long)(k - F.klo) * S.ny + j) * S.nx + i];
-  if (F.kind == SPARC_SRC_RANDOM) return F.f2d[(long long)j * S.nx + i] * __ldg(F.sdep + k);
-  return 0.0;
-}
-
-__device__ __forceinline__ double pulse_time(const SimDev &S, long long it) {
-  const ForcingDev &F = S.frc;
-  if (F.kind != SPARC_SRC_PULSE) return 0.0;
-  const double t = (double)it * F.timestep;
-  double T = F.amp_c * sin(2.0 * PI * (t - F.t1 + 2.0 * F.t0) / F.t0);
-  return T * exp(-1.0 * ((t - F.t1) * (t - F.t1)) / (2.0 * (F.st * F.st)));
-}
-
-// ------------------------------------------------------------ diagnostics
-// Block partial of the KE norm and the two minima, then the last CTA to
-// finish reduces all partials (no waiting: it is simply the last to arrive)
-// and applies the fail criterion of driver.f90:175-183.
-__device__ void diag_reduce(const SimDev &S, double ke, double mr, double mp) {
-  __shared__ double r[3][32];
-  __shared__ int am_last;
-  const int nt = blockDim.x * blockDim.y * blockDim.z;
-  const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5, nw = (nt + 31) >> 5;
-  const long long nb = (long long)gridDim.x * gridDim.y * gridDim.z;
-  const long long bid = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
-  for (int o = 16; o > 0; o >>= 1) {
-    ke += __shfl_down_sync(0xffffffffu, ke, o);
-    mr = fmin(mr, __shfl_down_sync(0xffffffffu, mr, o));
-    mp = fmin(mp, __shfl_down_sync(0xffffffffu, mp, o));
-  }
-  if (lane == 0) { r[0][warp] = ke; r[1][warp] = mr; r[2][warp] = mp; }
-  __syncthreads();
-  if (warp == 0) {
-    ke = lane < nw ? r[0][lane] : 0.0;
-    mr = lane < nw ? r[1][lane] : 1e300;
-    mp = lane < nw ? r[2][lane] : 1e300;
-    for (int o = 16; o > 0; o >>= 1) {
-      ke += __shfl_down_sync(0xffffffffu, ke, o);
-      mr = fmin(mr, __shfl_down_sync(0xffffffffu, mr, o));
-      mp = fmin(mp, __shfl_down_sync(0xffffffffu, mp, o));
-    }
-    if (lane == 0) {
-      S.partials[3 * bid] = ke;
-      S.partials[3 * bid + 1] = mr;
-      S.partials[3 * bid + 2] = mp;
-      __threadfence();
-      unsigned t = atomicAdd(S.counter, 1u);
-      am_last = (t == (unsigned)(nb - 1));
-    }
-  }
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  ke = 0.0; mr = 1e300; mp = 1e300;
-  for (long long b = tid; b < nb; b += nt) {
-    ke += __ldcg(S.partials + 3 * b);
-    mr = fmin(mr, __ldcg(S.partials + 3 * b + 1));
-    mp = fmin(mp, __ldcg(S.partials + 3 * b + 2));
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    ke += __shfl_down_sync(0xffffffffu, ke, o);
-    mr = fmin(mr, __shfl_down_sync(0xffffffffu, mr, o));
-    mp = fmin(mp, __shfl_down_sync(0xffffffffu, mp, o));
-  }
-  __syncthreads();
-  if (lane == 0) { r[0][warp] = ke; r[1][warp] = mr; r[2][warp] = mp; }
-  __syncthreads();
-  if (tid == 0) {
-    ke = 0.0; mr = 1e300; mp = 1e300;
-    for (int w = 0; w < nw; ++w) {
-      ke += r[0][w]; mr = fmin(mr, r[1][w]); mp = fmin(mp, r[2][w]);
-    }
-    const long long it = *S.iter;
-    // norm(): sqrt(sum/(nx*ny*nz)) (all_modules.f90:703), times dimc^2*dimrho
-    double nrm = sqrt(ke / ((double)S.nx * (double)S.ny * (double)S.nz));
-    double kev = nrm * S.dimc2rho;
-    S.diag[0] = kev;
-    S.diag[1] = mr;
-    S.diag[2] = mp;
-    S.diag[3] = (double)it;
-    // driver.f90:175-183; a NaN norm also counts as a failure
-    bool fail = !(kev <= 1000.0) || !(mr > 0.0) || !(mp > 0.0);
-    if (fail && *S.fail_iter < 0) *S.fail_iter = it;
-    *S.iter = it + 1;
-    *S.counter = 0u;
-  }
-}
-
-// ------------------------------------------------------------ helpers
-__device__ __forceinline__ int wrapi(int q, int n) {
-  q = q < 0 ? q + n : q;
-  return q >= n ? q - n : q;
-}
-
-// Global index of local tile position 0 along one axis.  Normally t0 - 5;
-// on a non-periodic axis the last tile may start closer than 6 points to
-// the edge, and its origin then moves down to n - 11 so that the one-sided
-// window f(n-11 .. n-1) is in the tile (interior points still see +-5).
-__device__ __forceinline__ int tile_origin(int t0, int T, int n, bool per) {
-  int o = t0 - 5;
-  if (!per && t0 + T >= n) o = min(o, n - 11);
-  return o;
-}
-
-// x or y derivative at local tile position from a row/column of shared
-// memory: `t(m)` returns the tile value at global index g0 + m.  Periodic
-// axes and interior points use the centred row (RHS bh = 5 / interior),
-// non-periodic edges the one-sided rows (derivatives.f90:72, 98).
-template <class Get>
-__device__ __forceinline__ double dxy(int q, int n, bool per, double sc,
-                                      Get t) {
-  double s = 0.0;
-  if (per || (q >= 5 && q < n - 5)) {
-#pragma unroll
-    for (int m = 0; m < 11; ++m) s += t(q - 5 + m) * c_dp[5][m];
-    return sc * s;
-  }
-  if (q < 5) {
-#pragma unroll
-    for (int m = 0; m < 11; ++m) s += t(m) * c_dp[q][m];
-    return sc * s;
-  }
-  const int row = n - 1 - q;
-#pragma unroll
-  for (int m = 0; m < 11; ++m) s += t(n - 1 - m) * c_dp[row][m];
-  return -sc * s;
-}
-
-// z derivative from the 11-deep window w (w[m] = f(base + m)), with the
-// bottom zero ghosts already in the window and the top one-sided rows
-// (derivatives.f90:509-545).
-__device__ __forceinline__ double dz(const double (&w)[11], int k, int nz,
-                                     double sc) {
-  double s = 0.0;
-  if (k < nz - 5) {
-#pragma unroll
-    for (int m = 0; m < 11; ++m) s += w[m] * c_dp[5][m];
-    return sc * s;
-  }
-  const int row = nz - 1 - k;
-#pragma unroll
-  for (int m = 0; m < 11; ++m) s += w[10 - m] * c_dp[row][m];
-  return -sc * s;
-}
-
-__device__ __forceinline__ void shift(double (&w)[11], double v) {
-#pragma unroll
-  for (int m = 0; m < 10; ++m) w[m] = w[m + 1];
-  w[10] = v;
-}
-
 // ------------------------------------------------ MP_QUIET_3D stage kernel
-// RHS.f90:18-175 fused with one RK stage of step.f90:26-61.
-template <int TX, int TY, int MODE, bool BG1D>
-__global__ void __launch_bounds__(TX *TY)
-    k_stage_quiet(const SimDev S, const double *__restrict__ a,
-                  const double *__restrict__ tin, double *__restrict__ so,
-                  double beta, double bnext, int zchunk) {
-  constexpr int HX = TX + 10, HY = TY + 10;
-  __shared__ double t_vx[HY][HX], t_vy[HY][HX], t_p[HY][HX];
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int nx = S.nx, ny = S.ny, nz = S.nz;
-  const long long N = S.N, NXY = (long long)nx * ny;
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
-  const int i = x0 + tx, j = y0 + ty;
-  const bool act = i < nx && j < ny;
-  const bool per = S.periodic;
-  const int k0 = blockIdx.z * zchunk, k1 = min(nz, k0 + zchunk);
-  const long long col = (long long)j * nx + i;
-  const long long it = *S.iter;
-  const double Tp = pulse_time(S, it);
-  const double dt = S.deltat;
-  const int gc = act ? S.colx[i] + S.bxdim * S.coly[j] : 0;
-  const int xo = tile_origin(x0, TX, nx, per), yo = tile_origin(y0, TY, ny, per);
-  const int cx0 = x0 - xo, cy0 = y0 - yo;  // interior offset in the tile
-
-  double wvz[11], wp[11];
-  const int b0 = min(k0 - 5, nz - 11);
-#pragma unroll
-  for (int m = 0; m < 11; ++m) {
-    const int kk = b0 + m;
-    const bool ok = act && kk >= 0;
-    const long long id = (long long)kk * NXY + col;
-    wvz[m] = ok ? __ldg(tin + 3 * N + id) : 0.0;
-    wp[m] = ok ? __ldg(tin + 4 * N + id) : 0.0;
-  }
+// One RK stage of the quiet equations (quiet_body.cuh): a block of 32 x 8
+// threads per (tile, z chunk), two per SM.  Layer ring: 30 KB a layer with
+// the uniform background (three layers), 40 KB with the 3-D one (two).
+template <bool BG1D>
+struct Quiet64 {
+  static constexpr int TY = 8, NS = BG1D ? 3 : 2;
+  using Buf = QuietBuf<double, TY, BG1D, NS, false>;
+};
+template <int MODE, bool BG1D>
+__global__ void __launch_bounds__(qg::TX *Quiet64<BG1D>::TY, 2)
+    k_quiet64(const SimDev S, const double *__restrict__ a, const double *__restrict__ tin,
+              double *__restrict__ so, double beta, double bnext, int zchunk) {
+  extern __shared__ __align__(16) double smem_q64[];
   double ke = 0.0, mr = 1e300, mp = 1e300;
+  const int k0 = blockIdx.z * zchunk;
+  quiet_body<double, Quiet64<BG1D>::TY, MODE, BG1D, Quiet64<BG1D>::NS>(
+      S, smem_q64, a, tin, so, beta, bnext, blockIdx.x * qg::TX, blockIdx.y * Quiet64<BG1D>::TY,
+      k0, min(S.nz, k0 + zchunk), threadIdx.x, threadIdx.y, ke, mr, mp);
+  if (MODE == F_LAST)
+    diag_reduce_t(S, ke, mr, mp,
+                  blockIdx.x + (long long)gridDim.x *
+                                   (blockIdx.y + (long long)gridDim.y * blockIdx.z),
+                  (long long)gridDim.x * gridDim.y * gridDim.z);
+}
 
-  for (int k = k0; k < k1; ++k) {
-    if (k > k0 && k <= nz - 6) {
-      const long long id = (long long)(k + 5) * NXY + col;
-      shift(wvz, act ? __ldg(tin + 3 * N + id) : 0.0);
-      shift(wp, act ? __ldg(tin + 4 * N + id) : 0.0);
-    }
-    const long long kb = (long long)k * NXY;
-    __syncthreads();
-    for (int t = tid; t < HY * HX; t += TX * TY) {
-      const int ly = t / HX, lx = t - ly * HX;
-      const bool inx = lx >= cx0 && lx < cx0 + TX, iny = ly >= cy0 && ly < cy0 + TY;
-      if (!inx && !iny) continue;
-      int gx = xo + lx, gy = yo + ly;
-      bool ok;
-      if (per) {
-        gx = wrapi(gx, nx);
-        gy = wrapi(gy, ny);
-        ok = true;
-      } else {
-        ok = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
-      }
-      const long long id = kb + (long long)gy * nx + gx;
-      if (iny) t_vx[ly][lx] = ok ? __ldg(tin + N + id) : 0.0;
-      if (inx) t_vy[ly][lx] = ok ? __ldg(tin + 2 * N + id) : 0.0;
-      t_p[ly][lx] = ok ? __ldg(tin + 4 * N + id) : 0.0;
-    }
-    __syncthreads();
-    if (!act) continue;
-    const long long id = kb + col;
-    double av[5], tv[5];
-#pragma unroll
-    for (int l = 0; l < 5; ++l) {
-      tv[l] = __ldg(tin + l * N + id);
-      av[l] = MODE == FIRST ? tv[l] : __ldg(a + l * N + id);
-    }
-    const double rho = tv[0], vx = tv[1], vy = tv[2], vz = tv[3], p = tv[4];
-    // derivatives (RHS.f90:42-48)
-    const int ry = cy0 + ty, rx = cx0 + tx;  // own tile row / column
-    double dvxdx = dxy(i, nx, per, S.stretchx, [&](int g) { return t_vx[ry][g - xo]; });
-    double gpx = dxy(i, nx, per, S.stretchx, [&](int g) { return t_p[ry][g - xo]; });
-    double dvydy = dxy(j, ny, per, S.stretchy, [&](int g) { return t_vy[g - yo][rx]; });
-    double gpy = dxy(j, ny, per, S.stretchy, [&](int g) { return t_p[g - yo][rx]; });
-    const double szk = __ldg(S.stretch + k);
-    double dvzdz = dz(wvz, k, nz, szk);
-    double gpz = dz(wp, k, nz, szk);
-    // CPML (RHS.f90:50-93); psi slots: 0 vz/vx/vy, 1 p
-    if (k < S.zb.np) {
-      const long long f = kb + col;
-      cpml<MODE>(S.zb, f, k, 1, beta, dt, gpz);
-      cpml<MODE>(S.zb, f, k, 0, beta, dt, dvzdz);
-    } else if (S.zt.on && k >= nz - S.zt.np) {
-      const int kl = k - (nz - S.zt.np);
-      const long long f = (long long)kl * NXY + col;
-      cpml<MODE>(S.zt, f, kl, 1, beta, dt, gpz);
-      cpml<MODE>(S.zt, f, kl, 0, beta, dt, dvzdz);
-    }
-    if (S.xb.on) {
-      if (i < S.xb.np) {
-        const long long f = i + (long long)S.xb.np * (j + (long long)ny * k);
-        cpml<MODE>(S.xb, f, i, 1, beta, dt, gpx);
-        cpml<MODE>(S.xb, f, i, 0, beta, dt, dvxdx);
-      } else if (i >= nx - S.xt.np) {
-        const int il = i - (nx - S.xt.np);
-        const long long f = il + (long long)S.xt.np * (j + (long long)ny * k);
-        cpml<MODE>(S.xt, f, il, 1, beta, dt, gpx);
-        cpml<MODE>(S.xt, f, il, 0, beta, dt, dvxdx);
-      }
-      if (j < S.yb.np) {
-        const long long f = i + (long long)nx * (j + (long long)S.yb.np * k);
-        cpml<MODE>(S.yb, f, j, 1, beta, dt, gpy);
-        cpml<MODE>(S.yb, f, j, 0, beta, dt, dvydy);
-      } else if (j >= ny - S.yt.np) {
-        const int jl = j - (ny - S.yt.np);
-        const long long f = i + (long long)nx * (jl + (long long)S.yt.np * k);
-        cpml<MODE>(S.yt, f, jl, 1, beta, dt, gpy);
-        cpml<MODE>(S.yt, f, jl, 0, beta, dt, dvydy);
-      }
-    }
-    // RHS algebra (RHS.f90:95-152)
-    const long long bi = BG1D ? (long long)k : id;
-    const double r0 = __ldg(S.rho0 + bi), ri = __ldg(S.rhoinv + bi),
-                 c2r = __ldg(S.c2rho0 + bi), grz = __ldg(S.grz + bi),
-                 gp0 = __ldg(S.gpz + bi), sg = __ldg(S.sponge + bi);
-    const double gk = __ldg(S.gblk + (long long)gc * nz + k);
-    const double div = dvxdx + dvydy + dvzdz;
-    double R[5];
-    R[0] = -grz * vz - r0 * div - sg * rho;
-    R[1] = -ri * gpx - sg * vx;
-    R[2] = -ri * gpy - sg * vy;
-    R[3] = -ri * (gpz + rho * gk) - vz * sg;
-    if (S.frc.kind != SPARC_SRC_NONE) {
-      const double frc = forcing_at(S, it, Tp, i, j, k);
-      if (S.frc.dir == 1) R[1] = R[1] + frc;
-      else if (S.frc.dir == 2) R[2] = R[2] + frc;
-      else R[3] = R[3] + frc;
-    }
-    R[4] = -c2r * div - vz * gp0 - sg * p;
-    // boundary planes (RHS.f90:154-164)
-    const bool zero = k == 0 || k == nz - 1 ||
-                      (!per && (i == 0 || i == nx - 1 || j == 0 || j == ny - 1));
-    // DAMPING: the velocity RHS minus the damping term after the boundary
-    // zeroing (RHS.f90:166-172), so the boundary planes move by -term
-    bool zl[5] = {zero, zero, zero, zero, zero};
-    if (S.term) {
-#pragma unroll
-      for (int l = 1; l < 4; ++l) {
-        R[l] = (zero ? 0.0 : R[l]) - __ldg(S.term + (long long)(l - 1) * N + id);
-        zl[l] = false;
-      }
-    }
-    if (MODE == LAST) {
-      double an[5];
-#pragma unroll
-      for (int l = 0; l < 5; ++l) {
-        an[l] = zl[l] ? av[l] : av[l] + dt * R[l];
-        so[l * N + id] = an[l];
-      }
-      const double p0v = __ldg(S.p0 + bi);
-      double m = (r0 + an[0]) * (an[1] * an[1] + an[2] * an[2] + an[3] * an[3]) / 2.0;
-      ke += m * m;
-      mr = fmin(mr, rho + r0);
-      mp = fmin(mp, p + p0v);
-    } else {
-#pragma unroll
-      for (int l = 0; l < 5; ++l) so[l * N + id] = zl[l] ? av[l] : av[l] + bnext * R[l];
+// Layers per z chunk of the quiet kernels: the extent with the least time,
+// where a block of zc layers costs zc + 2 layer times (its start and window
+// loads), an SM's resident blocks (two in FP64, three in FP32) share its
+// issue slots, and a lone block is bound by its own latency (1.3 of a
+// shared one's time).  At most 32 layers (256x256x300 FP32: 2.36 ms per
+// iteration at 24 and 32, 2.54 at 8; 64x64x128 FP64: 0.122 at the chosen 8,
+// 0.148 at 11 and 16, 0.133 at 4), and 8 with x/y CPML slabs, whose tiles
+// take longer than the others (133x117x171 FP64: 1.06 at 4 to 8, 1.13 at 16,
+// 1.27 at 25).
+static int quiet_zchunk(const Handle *h) {
+  const int occ = h->fp32 ? 3 : 2, zmax = h->use_hpml ? 8 : QUIET_ZMAX;
+  const long long tiles = (long long)((h->nx + 31) / 32) * ((h->ny + 7) / 8);
+  int best = std::min(h->nz, zmax);
+  double cost = 1e300;
+  for (int n = 1; n <= h->nz / 2; ++n) {
+    const int zc = (h->nz + n - 1) / n;
+    if (zc > zmax) continue;
+    const long long blocks = tiles * ((h->nz + zc - 1) / zc);
+    const long long full = blocks / (148 * occ), m = (blocks - full * 148 * occ + 147) / 148;
+    const double c = (zc + 2) * (full * occ + (m ? std::max<double>(m, 1.3) : 0.0));
+    if (c < cost) {
+      cost = c;
+      best = zc;
     }
   }
-  if (MODE == LAST) diag_reduce(S, ke, mr, mp);
+  return best;
 }
 
 int stage_geometry(Handle *h) {
-  // tile shape: (32, 8); the quiet kernel drops to (16, 8) on grids too
-  // small to fill the GPU.  The MHD kernels always use (32, 8).
-  h->tx = 32;
-  h->ty = 8;
-  long long tiles = (long long)((h->nx + h->tx - 1) / h->tx) *
-                    ((h->ny + h->ty - 1) / h->ty);
-  if (tiles < 64 && !h->magnetic) {
-    h->tx = 16;
-    tiles = (long long)((h->nx + 15) / 16) * ((h->ny + 7) / 8);
+  const long long tiles = (long long)((h->nx + 31) / 32) * ((h->ny + 7) / 8);
+  int zc;
+  if (h->magnetic) {
+    // about seven CTAs per SM on 148 SMs (one MHD CTA is resident per SM:
+    // shorter tails; each chunk pays 10 window warm-up layers), at most 40
+    // layers (swept 30..60 on the 256x256x300 flux tube in both precisions:
+    // 40 best, 60 1.5-2 % slower, 30 1-3 % slower)
+    const long long chunks = std::max<long long>(1, (148LL * 7 + tiles - 1) / tiles);
+    zc = (int)std::max<long long>(16, (h->nz + chunks - 1) / chunks);
+    zc = std::min(zc, 40);
+  } else {
+    zc = quiet_zchunk(h);
   }
-  // z chunk: about seven CTAs per SM on 148 SMs (one MHD CTA is resident per
-  // SM: shorter tails; each chunk pays 10 window warm-up layers)
-  const long long chunks = std::max<long long>(1, (148LL * 7 + tiles - 1) / tiles);
-  int zc = (int)std::max<long long>(16, (h->nz + chunks - 1) / chunks);
-  // MHD: at most 40 layers (swept 30..60 on the 256x256x300 flux tube in
-  // both precisions: 40 best, 60 1.5-2 % slower, 30 1-3 % slower)
-  if (h->magnetic) zc = std::min(zc, 40);
   zc = std::min(zc, h->nz);
   if (const char *kv = std::getenv("SPARC_ZCHUNK")) {  // A/B timing only
     const int v = std::atoi(kv);
-    if (v >= 11) zc = std::min(v, h->nz);
+    if (v >= 1) zc = std::min(v, h->nz);
   }
   h->zchunk = zc;
   h->max_stage_blocks = (int)(tiles * ((h->nz + zc - 1) / zc));
-  h->partials_blocks = (int)(tiles * ((h->nz + 10) / 11));
+  const int zmin = std::min(zc, 11);
+  h->partials_blocks = (int)(tiles * ((h->nz + zmin - 1) / zmin));
   return SPARC_OK;
 }
 
-template <int TX, int TY>
-static int launch_quiet(Handle *h, const SimDev &S, int stage,
-                        const double *a, const double *tin, double *so,
-                        cudaStream_t s) {
-  dim3 blk(TX, TY);
-  dim3 grd((h->nx + TX - 1) / TX, (h->ny + TY - 1) / TY,
-           (h->nz + h->zchunk - 1) / h->zchunk);
+static int launch_quiet(Handle *h, const SimDev &S, int stage, const double *a,
+                        const double *tin, double *so, cudaStream_t s) {
+  const int zc = std::min(h->zchunk, QUIET_ZMAX);
+  const dim3 blk(qg::TX, 8);
+  const dim3 grd((h->nx + qg::TX - 1) / qg::TX, (h->ny + 7) / 8, (h->nz + zc - 1) / zc);
   const double beta = h->betas[stage - 1];
   const double bnext = stage < 5 ? h->betas[stage] : h->deltat;
   const int mode = stage == 1 ? FIRST : (stage == 5 ? LAST : MID);
-#define QL(M, B) k_stage_quiet<TX, TY, M, B><<<grd, blk, 0, s>>>(S, a, tin, so, beta, bnext, h->zchunk)
+#define QL(M, B)                                                                          \
+  do {                                                                                    \
+    const int sm = (int)Quiet64<B>::Buf::bytes(zc);                                       \
+    cudaFuncSetAttribute(k_quiet64<M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm); \
+    k_quiet64<M, B><<<grd, blk, sm, s>>>(S, a, tin, so, beta, bnext, zc);                 \
+  } while (0)
   if (S.bg1d) {
-    if (mode == FIRST) QL(FIRST, true);
-    else if (mode == MID) QL(MID, true);
-    else QL(LAST, true);
+    if (mode == FIRST) QL(F_FIRST, true);
+    else if (mode == MID) QL(F_MID, true);
+    else QL(F_LAST, true);
   } else {
-    if (mode == FIRST) QL(FIRST, false);
-    else if (mode == MID) QL(MID, false);
-    else QL(LAST, false);
+    if (mode == FIRST) QL(F_FIRST, false);
+    else if (mode == MID) QL(F_MID, false);
+    else QL(F_LAST, false);
   }
 #undef QL
   return SPARC_OK;
@@ -689,22 +399,8 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
 int launch_stage(Handle *h, const SimDev &S, int stage, const double *a,
                  const double *tin, double *so, cudaStream_t s) {
   int r = SPARC_ERR_INVALID;
-  if (h->magnetic) {
-    if (h->tx != 32 || h->ty != 8) return SPARC_ERR_INVALID;
-    r = launch_mhd64p(h, S, stage, a, tin, so, s);
-    ++h->launches;
-    if (r == SPARC_OK && cudaGetLastError() != cudaSuccess) r = SPARC_ERR_CUDA;
-    return r;
-  }
-  const int key = h->tx * 100 + h->ty;
-#define DISPATCH(FN)                                            \
-  switch (key) {                                                \
-    case 3208: r = FN<32, 8>(h, S, stage, a, tin, so, s); break; \
-    case 1608: r = FN<16, 8>(h, S, stage, a, tin, so, s); break; \
-    default: r = SPARC_ERR_INVALID;                             \
-  }
-  DISPATCH(launch_quiet)
-#undef DISPATCH
+  r = h->magnetic ? launch_mhd64p(h, S, stage, a, tin, so, s)
+                  : launch_quiet(h, S, stage, a, tin, so, s);
   ++h->launches;
   if (r == SPARC_OK && cudaGetLastError() != cudaSuccess) r = SPARC_ERR_CUDA;
   return r;

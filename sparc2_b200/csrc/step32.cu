@@ -25,6 +25,7 @@
 
 #include "filter_body.cuh"
 #include "mhd_body.cuh"
+#include "quiet_body.cuh"
 #include "random_forcing.cuh"
 
 namespace sparc {
@@ -58,355 +59,33 @@ __device__ __forceinline__ float fcoef<float>(int t, int m) {
 using Sim32 = SimT<float>;
 using Face32 = FaceT<float>;
 
-// ------------------------------------------------------------- helpers
-__device__ __forceinline__ int wrap32(int q, int n) {
-  q = q < 0 ? q + n : q;
-  return q >= n ? q - n : q;
-}
-__device__ __forceinline__ int origin32(int t0, int T, int n, bool per) {
-  int o = t0 - 5;
-  if (!per && t0 + T >= n) o = min(o, n - 11);
-  return o;
-}
-
-template <int MODE>
-__device__ __forceinline__ void cpml32(const Face32 &F, long long f, int layer, int slot,
-                                       float beta, float dt, float &d) {
-  const long long pf = F.uniform ? (long long)layer : f;
-  const float pa = __ldg(F.pa + pf), pb = __ldg(F.pb + pf), pki = __ldg(F.pki + pf);
-  const long long o = (long long)slot * F.cnt + f;
-  const float v = F.vars[o];
-  float psi = v;
-  if (MODE != F_FIRST) psi = v + beta * F.scr[o];
-  const float rhs = pa * d + pb * psi;
-  d = d * pki + psi;
-  if (MODE == F_LAST) F.vars[o] = v + dt * rhs;
-  else F.scr[o] = rhs;
-}
-
-__device__ __forceinline__ float pulse_time32(const Sim32 &S, long long it) {
-  const ForcingT<float> &F = S.frc;
-  if (F.kind != SPARC_SRC_PULSE) return 0.f;
-  const double t = (double)it * F.timestep;
-  double T = F.amp_c * sin(2.0 * PI * (t - F.t1 + 2.0 * F.t0) / F.t0);
-  return (float)(T * exp(-1.0 * ((t - F.t1) * (t - F.t1)) / (2.0 * (F.st * F.st))));
-}
-
-__device__ __forceinline__ float forcing32(const Sim32 &S, float T, int i, int j, int k) {
-  const ForcingT<float> &F = S.frc;
-  if (F.kind == SPARC_SRC_PULSE)
-    return T * __ldg(F.fz + k) * (__ldg(F.fy + j) * __ldg(F.fx + i));
-  if (F.kind == SPARC_SRC_PSR && k >= F.klo && k < F.khi)
-    return F.psr[((long long)(k - F.klo) * S.ny + j) * S.nx + i];
-  if (F.kind == SPARC_SRC_RANDOM) return F.f2d[(long long)j * S.nx + i] * __ldg(F.sdep + k);
-  return 0.f;
-}
-
-template <class Get>
-__device__ __forceinline__ float dxy32(int q, int n, bool per, float sc, Get t) {
-  float s = 0.f;
-  if (per || (q >= 5 && q < n - 5)) {
-#pragma unroll
-    for (int m = 0; m < 11; ++m) s += t(q - 5 + m) * f_dp[5][m];
-    return sc * s;
-  }
-  if (q < 5) {
-#pragma unroll
-    for (int m = 0; m < 11; ++m) s += t(m) * f_dp[q][m];
-    return sc * s;
-  }
-  const int row = n - 1 - q;
-#pragma unroll
-  for (int m = 0; m < 11; ++m) s += t(n - 1 - m) * f_dp[row][m];
-  return -sc * s;
-}
-
-__device__ __forceinline__ float dz32(const float (&w)[11], int k, int nz, float sc) {
-  float s = 0.f;
-  if (k < nz - 5) {
-    const float d1 = w[6] - w[4], d2 = w[7] - w[3], d3 = w[8] - w[2], d4 = w[9] - w[1],
-                d5 = w[10] - w[0];
-    const float a = fmaf(f_dp[5][8], d3, fmaf(f_dp[5][10], d5, f_dp[5][6] * d1));
-    const float b = fmaf(f_dp[5][9], d4, f_dp[5][7] * d2);
-    return sc * (a + b);
-  }
-  const int row = nz - 1 - k;
-#pragma unroll
-  for (int m = 0; m < 11; ++m) s += w[10 - m] * f_dp[row][m];
-  return -sc * s;
-}
-
-__device__ __forceinline__ void shift32(float (&w)[11], float v) {
-#pragma unroll
-  for (int m = 0; m < 10; ++m) w[m] = w[m + 1];
-  w[10] = v;
-}
-
-// Per-CTA partial of the KE norm and minima (FP64) and the last-CTA
-// reduction with the fail criterion of driver.f90:175-183.
-// bid/nb: this block's index and the block count of the logical grid (a
-// stage split over several launches shares one logical grid).
-__device__ void diag_reduce32(const Sim32 &S, double ke, double mr, double mp, long long bid,
-                              long long nb) {
-  __shared__ double r[3][32];
-  __shared__ int am_last;
-  const int nt = blockDim.x * blockDim.y * blockDim.z;
-  const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5, nw = (nt + 31) >> 5;
-  for (int o = 16; o > 0; o >>= 1) {
-    ke += __shfl_down_sync(0xffffffffu, ke, o);
-    mr = fmin(mr, __shfl_down_sync(0xffffffffu, mr, o));
-    mp = fmin(mp, __shfl_down_sync(0xffffffffu, mp, o));
-  }
-  if (lane == 0) { r[0][warp] = ke; r[1][warp] = mr; r[2][warp] = mp; }
-  __syncthreads();
-  if (warp == 0) {
-    ke = lane < nw ? r[0][lane] : 0.0;
-    mr = lane < nw ? r[1][lane] : 1e300;
-    mp = lane < nw ? r[2][lane] : 1e300;
-    for (int o = 16; o > 0; o >>= 1) {
-      ke += __shfl_down_sync(0xffffffffu, ke, o);
-      mr = fmin(mr, __shfl_down_sync(0xffffffffu, mr, o));
-      mp = fmin(mp, __shfl_down_sync(0xffffffffu, mp, o));
-    }
-    if (lane == 0) {
-      S.partials[3 * bid] = ke;
-      S.partials[3 * bid + 1] = mr;
-      S.partials[3 * bid + 2] = mp;
-      __threadfence();
-      unsigned t = atomicAdd(S.counter, 1u);
-      am_last = (t == (unsigned)(nb - 1));
-    }
-  }
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  ke = 0.0; mr = 1e300; mp = 1e300;
-  for (long long b = tid; b < nb; b += nt) {
-    ke += __ldcg(S.partials + 3 * b);
-    mr = fmin(mr, __ldcg(S.partials + 3 * b + 1));
-    mp = fmin(mp, __ldcg(S.partials + 3 * b + 2));
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    ke += __shfl_down_sync(0xffffffffu, ke, o);
-    mr = fmin(mr, __shfl_down_sync(0xffffffffu, mr, o));
-    mp = fmin(mp, __shfl_down_sync(0xffffffffu, mp, o));
-  }
-  __syncthreads();
-  if (lane == 0) { r[0][warp] = ke; r[1][warp] = mr; r[2][warp] = mp; }
-  __syncthreads();
-  if (tid == 0) {
-    ke = 0.0; mr = 1e300; mp = 1e300;
-    for (int w = 0; w < nw; ++w) {
-      ke += r[0][w]; mr = fmin(mr, r[1][w]); mp = fmin(mp, r[2][w]);
-    }
-    const long long it = *S.iter;
-    double nrm = sqrt(ke / ((double)S.nx * (double)S.ny * (double)S.nz));
-    double kev = nrm * S.dimc2rho;
-    S.diag[0] = kev;
-    S.diag[1] = mr;
-    S.diag[2] = mp;
-    S.diag[3] = (double)it;
-    bool fail = !(kev <= 1000.0) || !(mr > 0.0) || !(mp > 0.0);
-    if (fail && *S.fail_iter < 0) *S.fail_iter = it;
-    *S.iter = it + 1;
-    *S.counter = 0u;
-  }
-}
-
 // ------------------------------------------ MP_QUIET_3D, precision form
-// RHS.f90:18-175 fused with one RK stage (as k_stage_quiet of step.cu),
-// FP32 with depth-scaled state.  Field scales: l = 0 rho, 1-3 v, 4 p.
-// The body covers the tile (x0, y0) of TX x TY columns over layers
-// [k0, k1); (tx, ty) is the calling thread's column in the tile.  Every
-// thread of the block calls it.  Diagnostics of the last stage accumulate
-// into ke, mr, mp.
-template <int TX, int TY, int MODE, bool BG1D>
-__device__ __forceinline__ void quiet_body(const Sim32 &S, const float *__restrict__ a,
-                                           const float *__restrict__ tin,
-                                           float *__restrict__ so, float beta, float bnext,
-                                           int x0, int y0, int k0, int k1, int tx, int ty,
-                                           float *zt, double &ke, double &mr, double &mp) {
-  constexpr int HX = TX + 10, HY = TY + 10;
-  __shared__ float t_vx[HY][HX], t_vy[HY][HX], t_p[HY][HX];
-  const int tid = ty * TX + tx;
-  const int nx = S.nx, ny = S.ny, nz = S.nz;
-  const long long N = S.N, NXY = (long long)nx * ny;
-  const int i = x0 + tx, j = y0 + ty;
-  const bool act = i < nx && j < ny;
-  const bool per = S.periodic;
-  const long long col = (long long)j * nx + i;
-  const long long it = *S.iter;
-  const float Tp = pulse_time32(S, it);
-  const float dt = (float)S.deltat;
-  const int gc = act ? S.colx[i] + S.bxdim * S.coly[j] : 0;
-  const int xo = origin32(x0, TX, nx, per), yo = origin32(y0, TY, ny, per);
-  const int cx0 = x0 - xo, cy0 = y0 - yo;
-  // depth scales of the layers this chunk touches, staged in shared memory
-  // (zt: 16 floats per layer, 1/sc of the 5 fields then sc)
-  const int zb = max(0, min(k0 - 5, nz - 11));
-  {
-    const int ze = min(nz, max(k1 + 5, zb + 11));
-    for (int t = tid; t < (ze - zb) * 16; t += TX * TY) {
-      const int kk = zb + (t >> 4), l = t & 15;
-      zt[t] = l < 5 ? S.isc[l * nz + kk] : (l >= 8 && l < 13 ? S.sc[(l - 8) * nz + kk] : 0.f);
-    }
-  }
-  __syncthreads();
-  auto isc_ = [&](int l, int kk) { return zt[(kk - zb) * 16 + l]; };
-  auto sc_ = [&](int l, int kk) { return zt[(kk - zb) * 16 + 8 + l]; };
-
-  float wvz[11], wp[11];  // physical values
-  const int b0 = min(k0 - 5, nz - 11);
-#pragma unroll
-  for (int m = 0; m < 11; ++m) {
-    const int kk = b0 + m;
-    const bool ok = act && kk >= 0;
-    const long long id = (long long)kk * NXY + col;
-    wvz[m] = ok ? __ldg(tin + 3 * N + id) * isc_(3, kk) : 0.f;
-    wp[m] = ok ? __ldg(tin + 4 * N + id) * isc_(4, kk) : 0.f;
-  }
-
-  for (int k = k0; k < k1; ++k) {
-    if (k > k0 && k <= nz - 6) {
-      const long long id = (long long)(k + 5) * NXY + col;
-      shift32(wvz, act ? __ldg(tin + 3 * N + id) * isc_(3, k + 5) : 0.f);
-      shift32(wp, act ? __ldg(tin + 4 * N + id) * isc_(4, k + 5) : 0.f);
-    }
-    const long long kb = (long long)k * NXY;
-    __syncthreads();
-    for (int t = tid; t < HY * HX; t += TX * TY) {
-      const int ly = t / HX, lx = t - ly * HX;
-      const bool inx = lx >= cx0 && lx < cx0 + TX, iny = ly >= cy0 && ly < cy0 + TY;
-      if (!inx && !iny) continue;
-      int gx = xo + lx, gy = yo + ly;
-      bool ok;
-      if (per) {
-        gx = wrap32(gx, nx);
-        gy = wrap32(gy, ny);
-        ok = true;
-      } else {
-        ok = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
-      }
-      const long long id = kb + (long long)gy * nx + gx;
-      if (iny) t_vx[ly][lx] = ok ? __ldg(tin + N + id) : 0.f;
-      if (inx) t_vy[ly][lx] = ok ? __ldg(tin + 2 * N + id) : 0.f;
-      t_p[ly][lx] = ok ? __ldg(tin + 4 * N + id) : 0.f;
-    }
-    __syncthreads();
-    if (!act) continue;
-    const long long id = kb + col;
-    float isv[5], scv[5];
-#pragma unroll
-    for (int l = 0; l < 5; ++l) {
-      isv[l] = isc_(l, k);
-      scv[l] = sc_(l, k);
-    }
-    float av[5], tv[5];
-#pragma unroll
-    for (int l = 0; l < 5; ++l) {
-      const float st = __ldg(tin + l * N + id);
-      av[l] = MODE == F_FIRST ? st : __ldg(a + l * N + id);
-      tv[l] = st * isv[l];
-    }
-    const float rho = tv[0], vx = tv[1], vy = tv[2], vz = tv[3], p = tv[4];
-    const int ry = cy0 + ty, rx = cx0 + tx;
-    const float sx = (float)S.stretchx, sy = (float)S.stretchy;
-    float dvxdx = isv[1] * dxy32(i, nx, per, sx, [&](int g) { return t_vx[ry][g - xo]; });
-    float gpx = isv[4] * dxy32(i, nx, per, sx, [&](int g) { return t_p[ry][g - xo]; });
-    float dvydy = isv[2] * dxy32(j, ny, per, sy, [&](int g) { return t_vy[g - yo][rx]; });
-    float gpy = isv[4] * dxy32(j, ny, per, sy, [&](int g) { return t_p[g - yo][rx]; });
-    const float szk = __ldg(S.stretch + k);
-    float dvzdz = dz32(wvz, k, nz, szk);
-    float gpz = dz32(wp, k, nz, szk);
-    if (k < S.zb.np) {
-      const long long f = kb + col;
-      cpml32<MODE>(S.zb, f, k, 1, beta, dt, gpz);
-      cpml32<MODE>(S.zb, f, k, 0, beta, dt, dvzdz);
-    } else if (S.zt.on && k >= nz - S.zt.np) {
-      const int kl = k - (nz - S.zt.np);
-      const long long f = (long long)kl * NXY + col;
-      cpml32<MODE>(S.zt, f, kl, 1, beta, dt, gpz);
-      cpml32<MODE>(S.zt, f, kl, 0, beta, dt, dvzdz);
-    }
-    if (S.xb.on) {
-      if (i < S.xb.np) {
-        const long long f = i + (long long)S.xb.np * (j + (long long)ny * k);
-        cpml32<MODE>(S.xb, f, i, 1, beta, dt, gpx);
-        cpml32<MODE>(S.xb, f, i, 0, beta, dt, dvxdx);
-      } else if (i >= nx - S.xt.np) {
-        const int il = i - (nx - S.xt.np);
-        const long long f = il + (long long)S.xt.np * (j + (long long)ny * k);
-        cpml32<MODE>(S.xt, f, il, 1, beta, dt, gpx);
-        cpml32<MODE>(S.xt, f, il, 0, beta, dt, dvxdx);
-      }
-      if (j < S.yb.np) {
-        const long long f = i + (long long)nx * (j + (long long)S.yb.np * k);
-        cpml32<MODE>(S.yb, f, j, 1, beta, dt, gpy);
-        cpml32<MODE>(S.yb, f, j, 0, beta, dt, dvydy);
-      } else if (j >= ny - S.yt.np) {
-        const int jl = j - (ny - S.yt.np);
-        const long long f = i + (long long)nx * (jl + (long long)S.yt.np * k);
-        cpml32<MODE>(S.yt, f, jl, 1, beta, dt, gpy);
-        cpml32<MODE>(S.yt, f, jl, 0, beta, dt, dvydy);
-      }
-    }
-    const long long bi = BG1D ? (long long)k : id;
-    const float r0 = __ldg(S.rho0 + bi), ri = __ldg(S.rhoinv + bi),
-                c2r = __ldg(S.c2rho0 + bi), grz = __ldg(S.grz + bi),
-                gp0 = __ldg(S.gpz + bi), sg = __ldg(S.sponge + bi);
-    const float gk = __ldg(S.gblk + (long long)gc * nz + k);
-    const float div = dvxdx + dvydy + dvzdz;
-    float R[5];
-    R[0] = -grz * vz - r0 * div - sg * rho;
-    R[1] = -ri * gpx - sg * vx;
-    R[2] = -ri * gpy - sg * vy;
-    R[3] = -ri * (gpz + rho * gk) - vz * sg;
-    if (S.frc.kind != SPARC_SRC_NONE) {
-      const float frc = forcing32(S, Tp, i, j, k);
-      if (S.frc.dir == 1) R[1] = R[1] + frc;
-      else if (S.frc.dir == 2) R[2] = R[2] + frc;
-      else R[3] = R[3] + frc;
-    }
-    R[4] = -c2r * div - vz * gp0 - sg * p;
-    const bool zero = k == 0 || k == nz - 1 ||
-                      (!per && (i == 0 || i == nx - 1 || j == 0 || j == ny - 1));
-    if (MODE == F_LAST) {
-      double an[5];
-#pragma unroll
-      for (int l = 0; l < 5; ++l) {
-        float c = S.carry[l * N + id];
-        const float t = zero ? av[l] : kahan(av[l], dt * (scv[l] * R[l]), c);
-        so[l * N + id] = t;
-        S.carry[l * N + id] = c;
-        an[l] = ((double)t - (double)c) * (double)isv[l];
-      }
-      const double p0v = __ldg(S.p0 + bi);
-      double m = ((double)r0 + an[0]) * (an[1] * an[1] + an[2] * an[2] + an[3] * an[3]) / 2.0;
-      ke += m * m;
-      mr = fmin(mr, (double)rho + (double)r0);
-      mp = fmin(mp, (double)p + p0v);
-    } else {
-#pragma unroll
-      for (int l = 0; l < 5; ++l)
-        so[l * N + id] = zero ? av[l] : av[l] + bnext * (scv[l] * R[l]);
-    }
-  }
-}
-
-template <int TX, int TY, int MODE, bool BG1D>
-__global__ void __launch_bounds__(TX *TY)
+// One RK stage of the quiet equations (quiet_body.cuh, depth-scaled state):
+// a block of 32 x 8 threads per (tile, z chunk), three per SM.  Layer ring
+// of three: 16 to 21 KB a layer (of two, 26 KB, for the last stage with the
+// 3-D background and the carries).
+template <int MODE, bool BG1D>
+struct Quiet32 {
+  static constexpr bool C = MODE == F_LAST;
+  static constexpr int TY = 8, NS = C && !BG1D ? 2 : 3, CTAS = 3;
+  using Buf = QuietBuf<float, TY, BG1D, NS, C>;
+};
+template <int MODE, bool BG1D>
+__global__ void __launch_bounds__(qg::TX *Quiet32<MODE, BG1D>::TY, Quiet32<MODE, BG1D>::CTAS)
     k_quiet32(const Sim32 S, const float *__restrict__ a, const float *__restrict__ tin,
               float *__restrict__ so, float beta, float bnext, int zchunk) {
-  extern __shared__ __align__(1024) float smem_raw32[];  // the depth-scale table
+  extern __shared__ __align__(16) float smem_q32[];
   double ke = 0.0, mr = 1e300, mp = 1e300;
   const int k0 = blockIdx.z * zchunk;
-  quiet_body<TX, TY, MODE, BG1D>(S, a, tin, so, beta, bnext, blockIdx.x * TX, blockIdx.y * TY,
-                                 k0, min(S.nz, k0 + zchunk), threadIdx.x, threadIdx.y, smem_raw32,
-                                 ke, mr, mp);
+  using Q = Quiet32<MODE, BG1D>;
+  quiet_body<float, Q::TY, MODE, BG1D, Q::NS>(S, smem_q32, a, tin, so, beta, bnext,
+                                              blockIdx.x * qg::TX, blockIdx.y * Q::TY, k0,
+                                              min(S.nz, k0 + zchunk), threadIdx.x, threadIdx.y,
+                                              ke, mr, mp);
   if (MODE == F_LAST)
-    diag_reduce32(S, ke, mr, mp,
-                  blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z),
+    diag_reduce_t(S, ke, mr, mp,
+                  blockIdx.x + (long long)gridDim.x *
+                                   (blockIdx.y + (long long)gridDim.y * blockIdx.z),
                   (long long)gridDim.x * gridDim.y * gridDim.z);
 }
 
@@ -680,17 +359,17 @@ Sim32 make_sim32(Handle *h) {
   return S;
 }
 
-template <int TX, int TY>
 static void launch_quiet32(Handle *h, const Sim32 &S, int mode, const float *a,
                            const float *tin, float *so, float beta, float bnext,
                            cudaStream_t s) {
-  dim3 blk(TX, TY);
-  dim3 grd((h->nx + TX - 1) / TX, (h->ny + TY - 1) / TY, (h->nz + h->zchunk - 1) / h->zchunk);
-  const int zsm = (h->zchunk + 16) * 16 * (int)sizeof(float);
-#define QL32(M, B)                                                                     \
-  do {                                                                                 \
-    cudaFuncSetAttribute(k_quiet32<TX, TY, M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, zsm); \
-    k_quiet32<TX, TY, M, B><<<grd, blk, zsm, s>>>(S, a, tin, so, beta, bnext, h->zchunk); \
+  const int zc = std::min(h->zchunk, QUIET_ZMAX);
+  const dim3 blk(qg::TX, 8);
+  const dim3 grd((h->nx + qg::TX - 1) / qg::TX, (h->ny + 7) / 8, (h->nz + zc - 1) / zc);
+#define QL32(M, B)                                                                        \
+  do {                                                                                    \
+    const int sm = (int)Quiet32<M, B>::Buf::bytes(zc);                                     \
+    cudaFuncSetAttribute(k_quiet32<M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm); \
+    k_quiet32<M, B><<<grd, blk, sm, s>>>(S, a, tin, so, beta, bnext, zc);                 \
   } while (0)
   if (S.bg1d) {
     if (mode == F_FIRST) QL32(F_FIRST, true);
@@ -765,8 +444,7 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
     }
 #undef ML32
   } else {
-    if (h->tx == 32) launch_quiet32<32, 8>(h, S, mode, a, tin, so, beta, bnext, s);
-    else launch_quiet32<16, 8>(h, S, mode, a, tin, so, beta, bnext, s);
+    launch_quiet32(h, S, mode, a, tin, so, beta, bnext, s);
   }
   ++h->launches;
   return cudaGetLastError() == cudaSuccess ? SPARC_OK : SPARC_ERR_CUDA;
@@ -907,7 +585,6 @@ __global__ void __launch_bounds__(BT, 1)
   __shared__ __align__(16) unsigned long long sS_raw[(sizeof(Sim32) + 7) / 8];
   __shared__ int s_w;
   float *smem = (float *)(((size_t)smem_raw32 + 127) & ~(size_t)127);
-  float *qzt = smem + 2 * MB::BUF + MB::XCH;  // quiet items' scale table
   Sim32 &sS = *reinterpret_cast<Sim32 *>(sS_raw);
   const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
   const int lo = PART == 1 ? counts[3] : 0, hi = PART == 0 ? counts[3] : counts[0];
@@ -944,11 +621,11 @@ __global__ void __launch_bounds__(BT, 1)
       mhd_body<float, MODE, false, false>(sS, nullptr, smem, a, tin, so, beta, bnext, x0, y0,
                                           k0, k1, 0, 0, ke, mr, mp);
     else if (sS.bg1d)
-      quiet_body<32, 16, MODE, true>(sS, a, tin, so, beta, bnext, x0, y0, k0, k1, threadIdx.x,
-                                     threadIdx.y + 8 * threadIdx.z, qzt, ke, mr, mp);
+      quiet_body<float, 16, MODE, true, MODE == F_LAST ? 2 : 3>(sS, smem, a, tin, so, beta, bnext, x0, y0, k0, k1,
+                                           threadIdx.x, threadIdx.y + 8 * threadIdx.z, ke, mr, mp);
     else
-      quiet_body<32, 16, MODE, false>(sS, a, tin, so, beta, bnext, x0, y0, k0, k1, threadIdx.x,
-                                      threadIdx.y + 8 * threadIdx.z, qzt, ke, mr, mp);
+      quiet_body<float, 16, MODE, false, 2>(sS, smem, a, tin, so, beta, bnext, x0, y0, k0, k1,
+                                            threadIdx.x, threadIdx.y + 8 * threadIdx.z, ke, mr, mp);
     if (MODE == F_LAST) batch_finish_step(L, sS, w, ke, mr, mp, tid);
     __syncthreads();
   }
@@ -1166,6 +843,10 @@ size_t batch_stage_smem() { return t32::MB::SMEM; }
 // 32 x 8 columns).
 static void launch_batch_stages(const BatchLaunch &B, cudaStream_t s) {
   const int sm = (int)t32::MB::smem_bytes(B.zmax);
+  static_assert(QuietBuf<float, 16, true, 2, true>::bytes(0) <= t32::MB::smem_bytes(0) &&
+                    QuietBuf<float, 16, true, 3, false>::bytes(0) <= t32::MB::smem_bytes(0) &&
+                    QuietBuf<float, 16, false, 2, true>::bytes(0) <= t32::MB::smem_bytes(0),
+                "the quiet items' ring fits the buffer of the MHD items");
   cudaFuncSetAttribute(k_batch_stage<F_FIRST, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   cudaFuncSetAttribute(k_batch_stage<F_MID, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   cudaFuncSetAttribute(k_batch_stage<F_LAST, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
