@@ -26,6 +26,7 @@ UNITS = {
     "noalloc.cu": [],
     "serve.cu": [],
     "damping.cu": [],
+    "state_io.cu": [],
 }
 HEADERS = ["internal.h", "mhd_body.cuh", "quiet_body.cuh", "random_forcing.cuh", "filter_body.cuh",
            "tmem_window.cuh", "tma_util.cuh"]

@@ -9,7 +9,6 @@
 #include <cstring>
 #include <new>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "internal.h"
@@ -310,20 +309,6 @@ static Handle::GraphEntry *graph_for(Handle *h, int fk) {
   return &h->graphs.back();
 }
 
-// f(i) for i in [0, n) on the host's cores (state conversion of the
-// precision form: one (field, layer) plane per index)
-template <class F>
-static void parallel_for(long long n, F f) {
-  const long long nt = std::max<long long>(
-      1, std::min<long long>(n, std::min(16u, std::max(1u, std::thread::hardware_concurrency()))));
-  std::vector<std::thread> th;
-  for (long long w = 0; w < nt; ++w)
-    th.emplace_back([=, &f] {
-      for (long long i = w; i < n; i += nt) f(i);
-    });
-  for (auto &t : th) t.join();
-}
-
 // Failure injection: one thread waits on an mbarrier that expects one
 // arrival which never comes; the bounded wait gives up after `polls` polls
 // or 10 ms of the global timer, whichever comes first, and raises the error
@@ -386,6 +371,7 @@ int sparc_create(const sparc_params *p, int device, sparc_handle **out) {
     delete h;
     return SPARC_ERR_CUDA;
   }
+  state_io_open();
   h->nx = p->nx; h->ny = p->ny; h->nz = p->nz;
   h->N = (long long)h->nx * h->ny * h->nz;
   h->magnetic = p->magnetic == 2;
@@ -469,7 +455,8 @@ int sparc_create(const sparc_params *p, int device, sparc_handle **out) {
   }
   for (int b = 0; !r && b < 3; ++b) {
     if (h->fp32) {
-      h->fbuf[b] = (float *)dev_alloc(h, (size_t)h->V * h->N * 4);
+      // (the free buffers hold half of the FP64 state each in state I/O)
+      h->fbuf[b] = (float *)dev_alloc(h, ((size_t)h->V * h->N + 1) / 2 * 8);
       if (!h->fbuf[b]) r = SPARC_ERR_NOMEM;
     } else {
       h->buf[b] = (double *)dev_alloc(h, (size_t)h->V * h->N * 8);
@@ -533,6 +520,7 @@ int sparc_destroy(sparc_handle *h) {
   drop_graphs(h);
   damping_destroy(h);
   for (void *p : h->allocs) cudaFree(p);
+  state_io_close();
   if (h->aux) cudaStreamSynchronize(h->aux);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   if (h->ev_join) cudaEventDestroy(h->ev_join);
@@ -560,9 +548,7 @@ int sparc_set_background(sparc_handle *h, const double *rho0,
   if (h->fp32) {
     r = setup32(h);
     if (r) return r;
-    h->h_scale.resize((size_t)2 * h->V * h->nz);
-    CK(h, cudaMemcpy(h->h_scale.data(), h->f_sc, h->h_scale.size() * 4,
-                     cudaMemcpyDeviceToHost));
+    h->scales_ready = true;
   } else {
     r = encode_tensor_maps(h);
     if (r) return r;
@@ -752,75 +738,13 @@ int sparc_sizes(const sparc_handle *h, int64_t *ns, int64_t *np) {
   return SPARC_OK;
 }
 
-// precision form: stored = float(sc * a), carry 0; a = (stored - carry)/sc
-static int set_state32(Handle *h, const double *a, const double *psi) {
-  const long long N = h->N;
-  const int nz = h->nz;
-  const long long NXY = (long long)h->nx * h->ny;
-  if (a && h->h_scale.empty()) return fail(h, SPARC_ERR_ORDER, "set the background first");
-  if (a) {
-    std::vector<float> t((size_t)h->V * N);
-    parallel_for((long long)h->V * nz, [&](long long lk) {
-      const double sc = h->h_scale[(size_t)lk];  // field l = lk / nz, layer lk % nz
-      const size_t o = (size_t)lk * NXY;
-      for (long long n = 0; n < NXY; ++n) t[o + n] = (float)(sc * a[o + n]);
-    });
-    // ordered on the handle's (non-blocking) stream, done before t goes
-    CK(h, cudaMemcpyAsync(h->fbuf[h->ra], t.data(), t.size() * 4, cudaMemcpyHostToDevice,
-                          h->stream));
-    CK(h, cudaMemsetAsync(h->f_carry, 0, t.size() * 4, h->stream));
-    CK(h, cudaStreamSynchronize(h->stream));
-  }
-  if (psi) {
-    size_t off = 0;
-    for (auto &F : h->f_faces)
-      if (F.on) {
-        std::vector<float> t(F.cnt * F.P);
-        for (size_t n = 0; n < t.size(); ++n) t[n] = (float)psi[off + n];
-        CK(h, cudaMemcpyAsync(F.vars, t.data(), t.size() * 4, cudaMemcpyHostToDevice,
-                              h->stream));
-        CK(h, cudaStreamSynchronize(h->stream));
-        off += t.size();
-      }
-  }
-  return SPARC_OK;
-}
-
-static int get_state32(Handle *h, double *a, double *psi) {
-  const long long N = h->N;
-  const int nz = h->nz, V = h->V;
-  const long long NXY = (long long)h->nx * h->ny;
-  CK(h, cudaStreamSynchronize(h->stream));
-  if (a) {
-    if (h->h_scale.empty()) return fail(h, SPARC_ERR_ORDER, "set the background first");
-    std::vector<float> t((size_t)V * N), c((size_t)V * N);
-    CK(h, cudaMemcpy(t.data(), h->fbuf[h->ra], t.size() * 4, cudaMemcpyDeviceToHost));
-    CK(h, cudaMemcpy(c.data(), h->f_carry, c.size() * 4, cudaMemcpyDeviceToHost));
-    parallel_for((long long)V * nz, [&](long long lk) {
-      const double isc = h->h_scale[(size_t)V * nz + (size_t)lk];
-      const size_t o = (size_t)lk * NXY;
-      for (long long n = 0; n < NXY; ++n) a[o + n] = ((double)t[o + n] - (double)c[o + n]) * isc;
-    });
-  }
-  if (psi) {
-    size_t off = 0;
-    for (auto &F : h->f_faces)
-      if (F.on) {
-        std::vector<float> t(F.cnt * F.P);
-        CK(h, cudaMemcpy(t.data(), F.vars, t.size() * 4, cudaMemcpyDeviceToHost));
-        for (size_t n = 0; n < t.size(); ++n) psi[off + n] = t[n];
-        off += t.size();
-      }
-  }
-  return SPARC_OK;
-}
-
 int sparc_set_state(sparc_handle *h, const double *a, const double *psi) {
   if (!h) return SPARC_ERR_INVALID;
   NOT_IN_BATCH(h);
   cudaSetDevice(h->device);
   // a restart from saved state clears the device error flag
   if (h->fp32) {
+    if (a && !h->scales_ready) return fail(h, SPARC_ERR_ORDER, "set the background first");
     CK(h, cudaStreamSynchronize(h->stream));
     const int r = set_state32(h, a, psi);
     if (r != SPARC_OK) return r;
@@ -828,18 +752,14 @@ int sparc_set_state(sparc_handle *h, const double *a, const double *psi) {
     CK(h, cudaStreamSynchronize(h->stream));
     return SPARC_OK;
   }
-  if (a)
-    CK(h, cudaMemcpyAsync(h->buf[h->ra], a, (size_t)h->V * h->N * 8,
-                          cudaMemcpyHostToDevice, h->stream));
-  if (psi) {
-    size_t off = 0;
+  int r;
+  if (a && (r = state_to_device(h, h->buf[h->ra], a, (size_t)h->V * h->N))) return r;
+  if (psi)
     for (auto &F : h->faces)
       if (F.on) {
-        CK(h, cudaMemcpyAsync(F.vars, psi + off, F.cnt * F.P * 8,
-                              cudaMemcpyHostToDevice, h->stream));
-        off += F.cnt * F.P;
+        if ((r = state_to_device(h, F.vars, psi, F.cnt * F.P))) return r;
+        psi += F.cnt * F.P;
       }
-  }
   CK(h, cudaMemsetAsync(h->d_err, 0, 4, h->stream));
   CK(h, cudaStreamSynchronize(h->stream));
   return SPARC_OK;
@@ -861,19 +781,19 @@ int sparc_get_state(sparc_handle *h, double *a, double *psi) {
   if (!h) return SPARC_ERR_INVALID;
   NOT_IN_BATCH(h);
   cudaSetDevice(h->device);
-  if (h->fp32) return get_state32(h, a, psi);
-  if (a)
-    CK(h, cudaMemcpyAsync(a, h->buf[h->ra], (size_t)h->V * h->N * 8,
-                          cudaMemcpyDeviceToHost, h->stream));
-  if (psi) {
-    size_t off = 0;
+  if (h->fp32) {
+    CK(h, cudaStreamSynchronize(h->stream));
+    if (a && !h->scales_ready) return fail(h, SPARC_ERR_ORDER, "set the background first");
+    return get_state32(h, a, psi);
+  }
+  int r;
+  if (a && (r = state_to_host(h, a, h->buf[h->ra], (size_t)h->V * h->N))) return r;
+  if (psi)
     for (auto &F : h->faces)
       if (F.on) {
-        CK(h, cudaMemcpyAsync(psi + off, F.vars, F.cnt * F.P * 8,
-                              cudaMemcpyDeviceToHost, h->stream));
-        off += F.cnt * F.P;
+        if ((r = state_to_host(h, psi, F.vars, F.cnt * F.P))) return r;
+        psi += F.cnt * F.P;
       }
-  }
   CK(h, cudaStreamSynchronize(h->stream));
   return SPARC_OK;
 }

@@ -280,7 +280,7 @@ struct Handle {
   float *fbuf[3] = {nullptr, nullptr, nullptr};
   float *f_carry = nullptr;
   float *f_sc = nullptr, *f_isc = nullptr;  // V x nz
-  std::vector<float> h_scale;               // host copy: sc then isc
+  bool scales_ready = false;                // f_sc, f_isc are set
   float *f_bg[FB_COUNT] = {};
   float *f_stretch = nullptr, *f_gblk = nullptr;
   FaceT<float> f_faces[6]{};
@@ -355,6 +355,15 @@ int source32(Handle *h);
 // batch.cu: the device slot of batch member h (null while the slot table
 // holding it has not been uploaded)
 int batch_member_slot(const Handle *h, const Slot32 **dslot);
+
+// state_io.cu: the state between host arrays (FP64) and the device; every
+// handle opens it once and closes it at its end
+void state_io_open();
+void state_io_close();
+int state_to_host(Handle *h, double *host, const void *dev, size_t count);
+int state_to_device(Handle *h, void *dev, const double *host, size_t count);
+int set_state32(Handle *h, const double *a, const double *psi);
+int get_state32(Handle *h, double *a, double *psi);
 
 // api.cu
 void *dev_alloc(Handle *h, size_t bytes);
