@@ -89,14 +89,6 @@ struct SimT {
 };
 using SimDev = SimT<double>;
 
-// z chunk boundaries of a persistent stage launch: chunk c covers layers
-// [b[c], b[c+1])
-struct ZSched {
-  static constexpr int MAX = 32;
-  int n;
-  int b[MAX + 1];
-};
-
 // PULSE = 2 forcing of the precision form: the per-layer pulse lists and
 // separable factors the forcing kernels read (all_modules.f90:521-663).
 struct Psr32 {

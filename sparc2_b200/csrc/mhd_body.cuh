@@ -587,17 +587,19 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       }
     }
     cp_commit_t();
-    // TMA copies of the layer, spread over warp 0 (lane l issues copies l
-    // and l + 32): copy c < 24 is own slot c (stage rho, a[0..7], 14
-    // background arrays, p0); with TH, copy 24 + s is halo plane s (state
-    // fields 1..7, then B0 x, y, z)
-    if (TMA && tid < 32) {
+    // TMA copies of the layer, spread over all warps (lane l of warp w issues
+    // copy 16 l + w; a warp that issued all of them held up every layer: FP64
+    // 256x256x300 12.58 -> 12.24 ms per iteration): copy c < 24 is own slot c
+    // (stage rho, a[0..7], 14 background arrays, p0); with TH, copy 24 + s is
+    // halo plane s (state fields 1..7, then B0 x, y, z).  Copies may complete
+    // before thread 0's expect: the phase ends with its arrival at the
+    // earliest.
+    if (TMA && tx < (TH ? 3 : 2)) {
       if (tid == 0) mbar_tx_t(&bar[b], own_bytes(k));
-      __syncwarp();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       R *ob = smem + b * BUF;
-      for (int c = tid; c < (TH ? NO + NH : NO); c += 32) {
-        if (skip_own(c, k)) continue;
+      const int c = tx * 16 + (tid >> 5);
+      if (c < (TH ? NO + NH : NO) && !skip_own(c, k)) {
         int map = mt, xx = x0, yy = y0, z = k;
         R *dst = ob + c * NC;
         if (c >= O_A && c < O_BG) {
@@ -635,9 +637,9 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   auto head = [&](int kk, R &v0, R &v1, R &v2) {
     const int id = kk * NXY + col;
     if (role == 0) {
-      v0 = __ldg(tin + 3 * N + id) * IS(3, kk);
-      v1 = __ldg(tin + 4 * N + id) * IS(4, kk);
-      v2 = __ldg(tin + 5 * N + id) * IS(5, kk);
+      v0 = __ldg(tin + 4 * N + id) * IS(4, kk);
+      v1 = __ldg(tin + 5 * N + id) * IS(5, kk);
+      v2 = __ldg(tin + 6 * N + id) * IS(6, kk);
     } else {
       const R iv = IS(1, kk);
       const R vx_ = __ldg(tin + N + id) * iv, vy_ = __ldg(tin + 2 * N + id) * iv,
@@ -645,7 +647,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       const R ox = __ldg(S.box + id), oy = __ldg(S.boy + id), oz = __ldg(S.boz + id);
       v0 = -vz_ * oy + vy_ * oz;
       v1 = -vx_ * oz + vz_ * ox;
-      v2 = __ldg(tin + 6 * N + id) * IS(6, kk);
+      v2 = vz_;
     }
   };
   // the z-window head of layer kk is read from DRAM a layer before it is
@@ -655,13 +657,13 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
     if (!act || kk >= nz) return;
     const int id = kk * NXY + col;
     if (role == 0) {
-      pf_l2(tin + 3 * N + id);
       pf_l2(tin + 4 * N + id);
       pf_l2(tin + 5 * N + id);
+      pf_l2(tin + 6 * N + id);
     } else {
       pf_l2(tin + N + id);
       pf_l2(tin + 2 * N + id);
-      pf_l2(tin + 6 * N + id);
+      pf_l2(tin + 3 * N + id);
       pf_l2(S.box + id);
       pf_l2(S.boy + id);
       pf_l2(S.boz + id);
@@ -838,33 +840,28 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       if (role == 0) {
         d0 = ip * DX(3); d5 = ib * DX(6); d7 = ib * DX(5);
         d1 = ip * DY(3); d4 = ib * DY(6); d8 = ib * DY(4);
-        d3 = DZ(0); d2 = DZ(1); d6 = DZ(2);
-        if (zpml) pz(1, 0, 2, d2, d3, d6);
+        d2 = DZ(0); d6 = DZ(1); d3 = DZ(2);
+        if (zpml) pz(1, 2, 3, d2, d6, d3);
         if (xpml) px(1, 3, 2, d0, d5, d7);
         if (ypml) py(1, 3, 2, d1, d4, d8);
-        X[cid] = d3;
-        // curl b: y and z components now, x after the exchange (fewer live
-        // registers across the barrier; the same arithmetic)
+        // curl b
+        d4 = d4 - d3;
         d5 = -d5 + d6;
         d7 = d7 - d8;
       } else {
         d0 = iv * DX(0); d2 = iv * DX(9); d3 = iv * DX(8);
         d1 = iv * DY(1); d4 = iv * DY(9); d5 = iv * DY(7);
         d6 = DZ(0); d7 = DZ(1); d8 = DZ(2);
-        if (zpml) pz(4, 5, 3, d7, d6, d8);
+        if (zpml) pz(4, 5, 0, d7, d6, d8);
         if (xpml) px(0, 4, 5, d0, d2, d3);
         if (ypml) py(0, 4, 5, d1, d4, d5);
-        X[NC + cid] = d8;
-        // curl(v x B0) and d(vx)/dx + d(vy)/dy now (fewer live registers
-        // across the barrier; the same arithmetic)
+        // curl(v x B0) and the divergence
         d4 = d4 - d7;
         d6 = d6 - d2;
         d3 = d3 - d5;
-        d0 = d0 + d1;
+        d0 = d0 + d1 + d8;
       }
     }
-    // the exchange involves only the role-0 and role-1 warps of rows ty
-    bar_pair_t(1 + ty);
     double an_rho = 0.0;
     if (act) {
       const bool zero = k == 0 || k == nz - 1 ||
@@ -877,8 +874,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       if (role == 0) {
         own_loads();
         const R ib = IS(5, k);
-        const R dzby = X[NC + cid];
-        const R cbx = d4 - dzby, cby = d5, cbz = d7;
+        const R cbx = d4, cby = d5, cbz = d7;
         const R c1 = cby * oz - cbz * oy, c2 = ox * cbz - cbx * oz, c3 = cbx * oy - cby * ox;
         const R ri = O(b, O_BG + B_RHOINV);
         R vxr = -ri * (d0 - (c1 * red)) - sg * vx;
@@ -934,8 +930,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
         if (MODE == F_LAST) VSQ[cid] = vsq;
       } else {
         const R p = Hv(3) * IS(4, k);
-        const R dvzdz = X[cid];
-        const R div = d0 + dvzdz;
+        const R div = d0;
         const R r0 = O(b, O_BG + B_RHO0);
         const R Rr = -O(b, O_BG + B_GRX) * vx - O(b, O_BG + B_GRY) * vy -
                          O(b, O_BG + B_GRZ) * vz - r0 * div - sg * rho;

@@ -231,18 +231,6 @@ int encode_tensor_maps(Handle *h) {
 
 // ------------------------- MP_MHD_3D, shared-body stage kernel
 
-// z chunk boundaries of the persistent launch: chunks of zchunk layers
-// (decreasing chunk sizes, so that the last items to start are short,
-// measured 1-3 % slower on the flux tube than equal chunks)
-static ZSched zsched(const Handle *h) {
-  ZSched Z{};
-  int n = 0;
-  for (int k = 0; k < h->nz && n < ZSched::MAX; k += h->zchunk) Z.b[n++] = k;
-  Z.b[n] = h->nz;
-  Z.n = n;
-  return Z;
-}
-
 // One FP64 MHD RK stage as a single persistent launch: each CTA (one per
 // SM) allocates its tensor memory once and pulls work items (32x8 tile, z
 // chunk) from a device counter until the list is done.  The edge/CPML
@@ -257,9 +245,9 @@ template <int MODE, bool TMA>
 __global__ void __launch_bounds__(mg::NT, 1)
     k_mhd64p(const SimDev S, const __grid_constant__ TmaSet T, const double *__restrict__ a,
              const double *__restrict__ tin, double *__restrict__ so, double beta,
-             double bnext, const ZSched Z, int mt, int ma, int ix0, int iy0, int nix, int nint,
+             double bnext, int zchunk, int mt, int ma, int ix0, int iy0, int nix, int nint,
              int ngen, const int2 *__restrict__ gen, unsigned *ctr) {
-  const int nch = Z.n;
+  const int nch = (S.nz + zchunk - 1) / zchunk;
   extern __shared__ __align__(1024) double smem_raw64[];
   double *smem = (double *)(((size_t)smem_raw64 + 127) & ~(size_t)127);
   __shared__ uint32_t s_tmem;
@@ -293,7 +281,7 @@ __global__ void __launch_bounds__(mg::NT, 1)
       x0 = (ix0 + t - ty * nix) * mg::TX;
       y0 = (iy0 + ty) * mg::TY;
     }
-    const int k0 = Z.b[c], k1 = Z.b[c + 1];
+    const int k0 = c * zchunk, k1 = min(S.nz, k0 + zchunk);
     // the body's first barrier orders every thread's read of s_w before
     // thread 0 takes the next item
     double ke = 0.0, mr = 1e300, mp = 1e300;
@@ -370,8 +358,7 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
     for (int n = 0; n < 24; ++n) T.m[n] = h->tmaps_ty[n];
   else
     std::memset(&T, 0, sizeof(T));
-  const ZSched Z = zsched(h);
-  const int nch = Z.n;
+  const int nch = (h->nz + h->zchunk - 1) / h->zchunk;
   const int nint = h->gnix * h->gniy;
   const long long total = (long long)(h->ngen + nint) * nch;
   const int grid = (int)std::min<long long>(h->pgrid, total);
@@ -380,7 +367,7 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
 #define MP64(M, U)                                                                           \
   do {                                                                                       \
     cudaFuncSetAttribute(k_mhd64p<M, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-    k_mhd64p<M, U><<<grid, blk, sm, s>>>(S, T, a, tin, so, beta, bnext, Z, mt, ma, h->gix0,   \
+    k_mhd64p<M, U><<<grid, blk, sm, s>>>(S, T, a, tin, so, beta, bnext, h->zchunk, mt, ma, h->gix0,   \
                                         h->giy0, h->gnix, nint, h->ngen, h->d_gen, ctr);     \
   } while (0)
   if (tma) {
