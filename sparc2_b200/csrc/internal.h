@@ -282,7 +282,7 @@ struct Handle {
   bool tma32 = false;
   bool allow_tma32 = true;   // FP32 MHD own-point loads by TMA (nx % 4 == 0)
   bool allow_tma64 = true;   // FP64 MHD own-point loads by TMA (nx even)
-  CUtensorMap tmaps32[18];
+  CUtensorMap tmaps32[24];  // as TmaSet (mhd_body.cuh)
 
   // member of a batch (sparc_batch_add): the batch owns the buffer roles,
   // the iteration and the stream order until sparc_batch_remove

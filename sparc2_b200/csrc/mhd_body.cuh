@@ -38,42 +38,36 @@ enum { B_RED, B_SPONGE, B_RHO0, B_GRX, B_GRY, B_GRZ, B_C2R, B_GPX, B_GPY,
        B_GPZ, B_RHOINV, B_CBX, B_CBY, B_CBZ };
 }  // namespace mg
 
-// shared-memory buffers of one layer (in R words, 128-byte multiple), the
-// exchange area and the dynamic size.  TH: the halo planes arrive as TMA
-// boxes (interior tiles of the plain form): a plane is 44 x 18 starting at
-// x0 - 6 (a 16-byte aligned start), each plane 128-byte aligned; otherwise
-// 42 x 18 copied by cp.async.  Exchange area:
-// d(vz)/dz and d(by)/dz in R, |v_new|^2 in FP64 (in the d(by)/dz slot in
-// the plain form, after its reader).
-template <class R, bool TH = false, bool HV = false>
+// shared-memory buffers of one layer (in R words, 128-byte multiple) and the
+// dynamic size.  TH: the halo planes arrive as TMA boxes, whose rows start at
+// a 16-byte aligned column (x0 - 6 in FP64, 44 wide; x0 - 8 in FP32, 48 wide),
+// each plane 128-byte aligned; otherwise 42 x 18 copied by cp.async.  The
+// precision form keeps |v_new|^2 of the last stage (FP64) after the buffers;
+// the plain form has it in the slot of a value already used.
+template <class R, bool TH = false>
 struct MhdBuf {
   static constexpr int ALIGN = 128 / (int)sizeof(R);
-  static_assert(!TH || sizeof(R) == 8, "TMA halo boxes in the plain form only");
-  static_assert(!HV || sizeof(R) == 4, "16-byte halo vectors in the precision form only");
-  // HV: halo rows of 48 values from x0 - 8 (a 16-byte aligned start), copied
-  // as 4-value vectors
-  static constexpr int HXL = TH ? 44 : (HV ? 48 : mg::HX);
-  static constexpr int XOFF = TH ? 1 : (HV ? 3 : 0);
-  static constexpr int HSL =
-      (TH || HV) ? (HXL * mg::HY + ALIGN - 1) / ALIGN * ALIGN : mg::HS;
+  static constexpr int HXL = TH ? (sizeof(R) == 8 ? 44 : 48) : mg::HX;
+  static constexpr int XOFF = TH ? (sizeof(R) == 8 ? 1 : 3) : 0;
+  static constexpr int HSL = TH ? (HXL * mg::HY + ALIGN - 1) / ALIGN * ALIGN : mg::HS;
   static constexpr int BUF = ((mg::NO * mg::NC + mg::NH * HSL) + ALIGN - 1) / ALIGN * ALIGN;
-  static constexpr int XCH = sizeof(R) == 4 ? 4 * mg::NC : 2 * mg::NC;
+  static constexpr int XCH = sizeof(R) == 4 ? 2 * mg::NC : 0;
   static constexpr size_t SMEM = (2 * (size_t)BUF + XCH) * sizeof(R) + 128;
   // plain form, general tiles: the per-lane and per-row coefficient tables
-  // follow the exchange area (dynamic, so one kernel can hold both bodies)
+  // follow (dynamic, so one kernel can hold both bodies)
   static constexpr size_t TABLES =
       (size_t)(mg::TX + mg::TY) * 11 * sizeof(R) + (mg::TX + mg::TY) * sizeof(int);
   static constexpr size_t SMEM_GEN = SMEM + (sizeof(R) == 8 ? TABLES : 0);
   // precision form: the depth scales (8 inverse, 8 forward per layer) of a
-  // chunk of at most zext layers follow the exchange area
+  // chunk of at most zext layers follow
   static constexpr size_t smem_bytes(int zext) {
     return SMEM + (sizeof(R) == 4 ? (size_t)(zext + 16) * 16 * sizeof(R) : 0);
   }
 };
 
 // tensor maps: [0..2] the state buffers (nx, ny, nz*V) and [3..17] the
-// background arrays in 32x8x1 boxes (own points); plain form: [18..20] the
-// state buffers and [21..23] B0 x, y, z in 44x18x1 halo boxes
+// background arrays in 32x8x1 boxes (own points); [18..20] the state buffers
+// and [21..23] B0 x, y, z in halo boxes (44x18x1 FP64, 48x18x1 FP32)
 struct TmaSet {
   CUtensorMap m[24];
 };
@@ -86,12 +80,6 @@ __device__ __forceinline__ void cp_r(R *dst, const R *src) {
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sm_addr_t(dst)), "l"(src)
                  : "memory");
-}
-// one 16-byte cp.async (both addresses 16-byte aligned)
-template <class R>
-__device__ __forceinline__ void cp16_t(R *dst, const R *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sm_addr_t(dst)), "l"(src)
-               : "memory");
 }
 __device__ __forceinline__ void cp_commit_t() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -121,6 +109,15 @@ __device__ __forceinline__ int origin_t(int t0, int T, int n, bool per) {
   int o = t0 - 5;
   if (!per && t0 + T >= n) o = min(o, n - 11);
   return o;
+}
+
+// the same where the halo rows are TMA boxes: the box starts XOFF columns
+// earlier, at a multiple of 16 bytes (n is even in FP64, a multiple of 4 in
+// FP32, so n - 12 and n - 16 are)
+template <class R>
+__host__ __device__ __forceinline__ int origin_th(int t0, int T, int n) {
+  const int o = t0 - 5, e = sizeof(R) == 8 ? n - 11 : n - 13;
+  return t0 + T >= n && e < o ? e : o;
 }
 
 template <class R>
@@ -368,7 +365,7 @@ inline void mhd_interior_rect(int nx, int ny, const int np[4], int &ix0, int &ix
 // (tmem_window.cuh; tw is this warp's window address, the caller allocates
 // and frees): each layer loads them, shifts in the new head, stores them
 // back and forms the z derivatives, so they hold registers only then.
-template <class R, int MODE, bool TMA, bool INT, bool TW = false>
+template <class R, int MODE, bool TMA, bool INT, bool TH, bool TW = false>
 __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *smem,
                                          const R *__restrict__ a,
                                          const R *__restrict__ tin,
@@ -377,16 +374,8 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
                                          double &ke, double &mr, double &mp, uint32_t tw = 0) {
   static_assert(!TW || sizeof(R) == 8, "TMEM windows of FP64 values");
   using namespace mg;
-  // halo planes by TMA in the plain form's interior kernel (measured: 4 %
-  // faster in FP64; in FP32 the 48-wide boxes cost more than the cp.async
-  // copies they replace)
-  constexpr bool TH = TMA && INT && sizeof(R) == 8;
-  // precision form, interior tiles of a grid whose rows are 16-byte
-  // multiples (the TMA own-point condition): halo rows of 48 values from
-  // x0 - 8 copied as 16-byte vectors, 216 of them per plane, one per role-1
-  // thread, in place of one 4-byte copy per halo position
-  constexpr bool HV = TMA && INT && sizeof(R) == 4;
-  using MB = MhdBuf<R, TH, HV>;
+  static_assert(TMA || !TH, "halo boxes come with the own-point boxes");
+  using MB = MhdBuf<R, TH>;
   constexpr int BUF = MB::BUF, HXL = MB::HXL, XOFF = MB::XOFF, HSL = MB::HSL;
   constexpr bool SCALED = sizeof(R) == 4;
   __shared__ unsigned long long bar[2];
@@ -398,7 +387,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   const bool act = INT || (i < nx && j < ny);
   const bool per = S.periodic;
   const int col = j * nx + i;
-  const int xo = INT ? x0 - 5 : origin_t(x0, TX, nx, per);
+  const int xo = INT ? x0 - 5 : (TH ? origin_th<R>(x0, TX, nx) : origin_t(x0, TX, nx, per));
   const int yo = INT ? y0 - 5 : origin_t(y0, TY, ny, per);
   const int ry = y0 - yo + ty, rx = x0 - xo + tx;
   const int own = ry * HXL + rx + XOFF;
@@ -426,12 +415,12 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   // window start in the tile, so every x/y derivative is one branch-free
   // sum: the centred row; one-sided row q at the low edge (q = i); at the
   // high edge -row q reversed over f(n-11..n-1) (derivatives.f90:72, 98).
-  // CTA-uniform: every lane's (row's) stencil is the centred one (periodic
-  // axis, or no lane within 5 points of an edge); then the centred sum
-  // from the window start cxo (cyo) of lane (row) 0 serves
+  // Where every lane of the tile (this row, a warp) has the centred stencil
+  // (periodic axis, or no point within 5 of an edge), the centred sum
+  // serves, from the window start cxo of lane 0
   const bool cen_x = per || (x0 >= 5 && x0 + TX <= nx - 5);
-  const bool cen_y = per || (y0 >= 5 && y0 + TY <= ny - 5);
-  const int cxo = x0 - 5 - xo, cyo = y0 - 5 - yo;
+  const bool cen_y = per || (j >= 5 && j < ny - 5);
+  const int cxo = x0 - 5 - xo;
   // the tables: FP64 in the dynamic buffer after the exchange area
   // (MhdBuf::SMEM_GEN), FP32 static (its depth scales follow the exchange
   // area)
@@ -441,7 +430,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   R *cxs = cxs_s, *cys = cys_s;
   int *cxb = cxb_s, *cyb = cyb_s;
   if constexpr (DYN_T) {
-    cxs = smem + 2 * BUF + MB::XCH;
+    cxs = smem + 2 * BUF;
     cys = cxs + TX * 11;
     cxb = reinterpret_cast<int *>(cys + TY * 11);
     cyb = cxb + TX;
@@ -474,27 +463,21 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   __syncthreads();
   auto O = [&](int b, int slot) -> R { return smem[b * BUF + slot * NC + cid]; };
   auto Hp = [&](int b, int slot) -> R * { return smem + b * BUF + NO * NC + slot * HSL; };
-  R *X = smem + 2 * BUF;
+  // |v_new|^2 of the last stage (role 0 writes, role 1 reads after a barrier);
+  // plain form: in the slot of a[1], which its writer has read
+  auto VSQ = [&](int b) -> double & {
+    if constexpr (SCALED) return reinterpret_cast<double *>(smem + 2 * BUF)[cid];
+    else return reinterpret_cast<double *>(smem + b * BUF)[(O_A + 1) * NC + cid];
+  };
+  // Halo positions a thread copies (without TMA halos) and turns into fluxes:
+  // role 0 its own column, whose B0 it keeps for the momentum equations;
+  // role 1 the 400 positions around the tile that a stencil reads (ten rows
+  // of 32, then ten columns of 8), one or two per thread.
   int hs0 = -1, hs1 = -1, ho0 = 0, ho1 = 0;
   {
     const int cx0 = x0 - xo, cy0 = y0 - yo;
-    auto pos = [&](int t, int &hs, int &ho) {
-      if constexpr (HV) {  // vector t of 216: row t / 12, values 4 (t % 12) ..
-        if (t >= HY * (HXL / 4)) return;
-        const int ly = t / (HXL / 4), lx = (t - ly * (HXL / 4)) * 4;
-        const int gx = x0 - 8 + lx, gy = yo + ly;
-        // inside the grid by the interior test (x0 >= 32, x0 + 40 <= nx
-        // with nx a multiple of 4); checked so that no copy can leave it
-        if (gx < 0 || gx + 3 >= nx || gy < 0 || gy >= ny) return;
-        hs = ly * HXL + lx;
-        ho = gy * nx + gx;
-        return;
-      }
-      if (t >= HS) return;
-      const int ly = t / HX, lx = t - ly * HX;
-      const bool inx = lx >= cx0 && lx < cx0 + TX, iny = ly >= cy0 && ly < cy0 + TY;
-      if (!inx && !iny) return;
-      if (TH) {  // in the domain by the interior test; no global offset
+    auto pos = [&](int lx, int ly, int &hs, int &ho) {
+      if (TH) {  // zero outside the grid; no offset needed
         hs = ly * HXL + lx + XOFF;
         return;
       }
@@ -502,20 +485,22 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       if (per) {
         gx = wrap_t(gx, nx);
         gy = wrap_t(gy, ny);
-      } else if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) {
-        return;
       }
-      hs = t;
+      if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) return;
+      hs = ly * HXL + lx;
       ho = gy * nx + gx;
     };
-    // halo positions 0..511 one per thread, 512..755 on role 1 (role 0
-    // carries the TMA issue and the heavier momentum update); HV: the
-    // vectors on role 1
-    if constexpr (HV) {
-      if (role == 1) pos(tid - NC, hs0, ho0);
+    auto yrow = [&](int h, int &hs, int &ho) { pos(rx, h < cy0 ? h : h + TY, hs, ho); };
+    if (role == 0) {
+      pos(rx, ry, hs0, ho0);
     } else {
-      pos(tid, hs0, ho0);
-      if (role == 1) pos(tid + NC, hs1, ho1);
+      yrow(ty, hs0, ho0);
+      if (ty < 2) {
+        yrow(8 + ty, hs1, ho1);
+      } else if (cid < 64 + 10 * TY) {
+        const int q = cid - 64, r = q / 10, c = q - r * 10;
+        pos(c < cx0 ? c : c + TX, cy0 + r, hs1, ho1);
+      }
     }
   }
   // Own-point arrays not read: where the sponge vanishes outside the CPML
@@ -540,16 +525,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   };
   auto issue = [&](int k, int b) {
     const int kb = k * NXY;
-    if (HV && hs0 >= 0) {
-      R *h = Hp(b, 0) + hs0;
-      const int id = kb + ho0;
-#pragma unroll
-      for (int sl = 0; sl < 7; ++sl) cp16_t(h + sl * HSL, tin + (sl + 1) * N + id);
-      cp16_t(h + 7 * HSL, S.box + id);
-      cp16_t(h + 8 * HSL, S.boy + id);
-      cp16_t(h + 9 * HSL, S.boz + id);
-    }
-    if (!TH && !HV && hs0 >= 0) {
+    if (!TH && hs0 >= 0) {
       R *h = Hp(b, 0) + hs0;
       const int id = kb + ho0;
 #pragma unroll
@@ -610,8 +586,8 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
         } else if (c >= NO) {
           const int sl = c - NO;
           dst = Hp(b, sl);
-          xx = x0 - 5 - XOFF;
-          yy = y0 - 5;
+          xx = xo - XOFF;
+          yy = yo;
           if (sl < 7) {
             map = 18 + mt;
             z = (sl + 1) * nz + k;
@@ -625,34 +601,50 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   };
   // fluxes v x B0 (stored velocity units) in place of the B0 halo values,
   // at the halo positions this thread copied
-  auto flux = [&](int b, int t) {
+  auto flux = [&](int b, int t, R &bx0, R &by0, R &bz0) {
     R *H = Hp(b, 0) + t;
     const R vx_ = H[0], vy_ = H[HSL], vz_ = H[2 * HSL];
-    const R bx0 = H[7 * HSL], by0 = H[8 * HSL], bz0 = H[9 * HSL];
+    bx0 = H[7 * HSL];
+    by0 = H[8 * HSL];
+    bz0 = H[9 * HSL];
     H[7 * HSL] = -vz_ * by0 + vy_ * bz0;
     H[8 * HSL] = -vx_ * bz0 + vz_ * bx0;
     H[9 * HSL] = -vy_ * bx0 + vx_ * by0;
   };
   R w0[11], w1[11], w2[11];  // physical values
-  auto head = [&](int kk, R &v0, R &v1, R &v2) {
+  // The values a window head of layer kk is made of, and the head: momentum
+  // p, bx, by; the other role the fluxes v x B0 (1 and 2) and vz.
+  R q[6];
+  auto head_load = [&](int kk) {
     const int id = kk * NXY + col;
     if (role == 0) {
-      v0 = __ldg(tin + 4 * N + id) * IS(4, kk);
-      v1 = __ldg(tin + 5 * N + id) * IS(5, kk);
-      v2 = __ldg(tin + 6 * N + id) * IS(6, kk);
+      q[0] = __ldg(tin + 4 * N + id);
+      q[1] = __ldg(tin + 5 * N + id);
+      q[2] = __ldg(tin + 6 * N + id);
+    } else {
+      q[0] = __ldg(tin + N + id);
+      q[1] = __ldg(tin + 2 * N + id);
+      q[2] = __ldg(tin + 3 * N + id);
+      q[3] = __ldg(S.box + id);
+      q[4] = __ldg(S.boy + id);
+      q[5] = __ldg(S.boz + id);
+    }
+  };
+  auto head_make = [&](int kk, R &v0, R &v1, R &v2) {
+    if (role == 0) {
+      v0 = q[0] * IS(4, kk);
+      v1 = q[1] * IS(5, kk);
+      v2 = q[2] * IS(6, kk);
     } else {
       const R iv = IS(1, kk);
-      const R vx_ = __ldg(tin + N + id) * iv, vy_ = __ldg(tin + 2 * N + id) * iv,
-                  vz_ = __ldg(tin + 3 * N + id) * iv;
-      const R ox = __ldg(S.box + id), oy = __ldg(S.boy + id), oz = __ldg(S.boz + id);
-      v0 = -vz_ * oy + vy_ * oz;
-      v1 = -vx_ * oz + vz_ * ox;
+      const R vx_ = q[0] * iv, vy_ = q[1] * iv, vz_ = q[2] * iv;
+      v0 = -vz_ * q[4] + vy_ * q[5];
+      v1 = -vx_ * q[5] + vz_ * q[3];
       v2 = vz_;
     }
   };
-  // the z-window head of layer kk is read from DRAM a layer before it is
-  // needed; an L2 prefetch two layers earlier takes that latency off the
-  // layer loop
+  // the head of layer kk + 5 is loaded a layer before layer kk needs it (into
+  // q), and brought into L2 two layers before that
   auto prefetch = [&](int kk) {
     if (!act || kk >= nz) return;
     const int id = kk * NXY + col;
@@ -671,14 +663,20 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   };
   issue(k0, 0);
   prefetch(k0 + 6);
+  prefetch(k0 + 7);
   {
     const int b0 = min(k0 - 5, nz - 11);
 #pragma unroll
     for (int m = 0; m < 11; ++m) {
       const int kk = b0 + m;
-      if (act && kk >= 0) head(kk, w0[m], w1[m], w2[m]);
-      else w0[m] = w1[m] = w2[m] = R(0);
+      if (act && kk >= 0) {
+        head_load(kk);
+        head_make(kk, w0[m], w1[m], w2[m]);
+      } else {
+        w0[m] = w1[m] = w2[m] = R(0);
+      }
     }
+    if (act && k0 + 1 < k1 && k0 + 1 <= nz - 6) head_load(k0 + 6);
     if constexpr (TW) {
       __syncwarp();
       tm_wait_st();  // a previous work item's stores to these columns
@@ -695,16 +693,27 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   const R *gcol = S.gblk + (act ? S.colx[i] + S.bxdim * S.coly[j] : 0) * nz;
   // PULSE = 1 time factor: the iteration is fixed during a stage
   const R Tp = S.frc.kind == SPARC_SRC_PULSE ? pulse_time_t(S, *S.iter) : R(0);
-  // |v_new|^2 of the last stage (role 0 writes, role 1 reads after a barrier)
-  double *VSQ = (double *)(SCALED ? X + 2 * NC : X + NC);
+
+  // x/y CPML slabs of this column
+  const bool xbot = i < S.xb.np, ybot = j < S.yb.np;
+  const bool xpml = !INT && S.xb.on && act && (xbot || i >= nx - S.xt.np);
+  const bool ypml = !INT && S.yb.on && act && (ybot || j >= ny - S.yt.np);
+  auto face_x = [&](int k) -> long long {
+    const int np = xbot ? S.xb.np : S.xt.np;
+    return (xbot ? i : i - (nx - np)) + (long long)np * (j + (long long)ny * k);
+  };
+  auto face_y = [&](int k) -> long long {
+    const int np = ybot ? S.yb.np : S.yt.np;
+    return i + (long long)nx * ((ybot ? j : j - (ny - np)) + (long long)np * k);
+  };
 
   for (int k = k0; k < k1; ++k) {
     const int b = (k - k0) & 1;
     const int id = k * NXY + col;
     R h0 = 0, h1 = 0, h2 = 0;
     const bool sh = k > k0 && k <= nz - 6;
-    if (sh && act) head(k + 5, h0, h1, h2);
-    prefetch(k + 7);
+    if (sh && act) head_make(k + 5, h0, h1, h2);
+    prefetch(k + 8);
     // precision form, last stage: the compensation carries of layer k + 2
     // into L2 (they are read just before their use)
     if (SCALED && MODE == F_LAST && act && k + 2 < k1) {
@@ -721,21 +730,32 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
         pf_l2(S.carry + 7 * N + id2);
       }
     }
-    // momentum role: own-point B0 (its halo slots will hold the fluxes),
-    // gravity and forcing, prefetched into L1 here and loaded after the
-    // exchange barrier (not live across the derivatives: fewer registers)
-    R ox = 0, oy = 0, oz = 0, gk = 0, frc = 0;
-    auto own_loads = [&] {
-      ox = __ldg(S.box + id);
-      oy = __ldg(S.boy + id);
-      oz = __ldg(S.boz + id);
-      gk = __ldg(gcol + k);
-      if (S.frc.kind != SPARC_SRC_NONE) frc = forcing_t(S, Tp, i, j, k);
-    };
-    if (role == 0 && act) {
-      pf_l1(S.box + id);
-      pf_l1(S.boy + id);
-      pf_l1(S.boz + id);
+    // the CPML fields and profiles of this layer's point into L1: their
+    // latency was a sixth of a layer's time in the tiles that have them
+    const bool zpml = S.zb.on && (k < S.zb.np || k >= nz - S.zt.np);
+    if (!INT || zpml) {
+      auto pf_face = [&](const FaceT<R> &F, long long f, int layer, int s0, int s1, int s2) {
+        const long long pf = F.uniform ? (long long)layer : f;
+        pf_l1(F.pa + pf);
+        pf_l1(F.pb + pf);
+        pf_l1(F.pki + pf);
+        const int sl[3] = {s0, s1, s2};
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          pf_l1(F.vars + (long long)sl[m] * F.cnt + f);
+          if (MODE != F_FIRST) pf_l1(F.scr + (long long)sl[m] * F.cnt + f);
+        }
+      };
+      if (zpml && act) {
+        const bool bot = k < S.zb.np;
+        const int kl = bot ? k : k - (nz - S.zt.np);
+        pf_face(bot ? S.zb : S.zt, (long long)kl * NXY + col, kl, role ? 4 : 1, role ? 5 : 2,
+                role ? 0 : 3);
+      }
+      if (xpml) pf_face(xbot ? S.xb : S.xt, face_x(k), 0, role ? 0 : 1, role ? 4 : 3,
+                        role ? 5 : 2);
+      if (ypml) pf_face(ybot ? S.yb : S.yt, face_y(k), 0, role ? 0 : 1, role ? 4 : 3,
+                        role ? 5 : 2);
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     const R szk = __ldg(S.stretch + k);
@@ -765,18 +785,17 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
     // TH: every thread waits for the layer's TMA copies (its flux positions
     // arrive that way); otherwise thread 0 alone, before the barrier
     if (TH) mine = mbar_wait_t(&bar[b], (phase >> b) & 1u, S.err);
-    if constexpr (HV) {
-      if (mine && hs0 >= 0)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) flux(b, hs0 + q);
-    } else {
-      if (mine && hs0 >= 0) flux(b, hs0);
-      if (mine && hs1 >= 0) flux(b, hs1);
+    R ox = 0, oy = 0, oz = 0;  // role 0: B0 of its column
+    if (mine && hs0 >= 0) flux(b, hs0, ox, oy, oz);
+    if (mine && hs1 >= 0) {
+      R u0, u1, u2;
+      flux(b, hs1, u0, u1, u2);
     }
     if (TMA && !TH && tid == 0) mine = mbar_wait_t(&bar[b], (phase >> b) & 1u, S.err);
     phase ^= 1u << b;
     if (!__syncthreads_and(mine)) { ok = false; break; }
     if (k + 1 < k1) issue(k + 1, b ^ 1);
+    if (act && k + 1 < k1 && k + 1 <= nz - 6) head_load(k + 6);
     if constexpr (!TW) {
       if (sh) { shift_t(w0, h0); shift_t(w1, h1); shift_t(w2, h2); }
     }
@@ -789,29 +808,56 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
         return dz_t(w2, k, nz, szk);
       }
     };
-    auto DX = [&](int slot) {
-      const R *row = Hp(b, slot) + ry * HXL + XOFF;
-      if (INT) return sx * csum_t(row + tx, 1);
-      if (cen_x) return sx * csum_t(row + cxo + tx, 1);
-      const R *r = row + cxb[tx], *c = cxs + tx * 11;
-      R sum = R(0);
+    // x (y) derivatives of three planes; one-sided tiles take each
+    // coefficient once for the three
+    auto DX = [&](int s0, int s1, int s2, R &e0, R &e1, R &e2) {
+      const R *r0 = Hp(b, s0) + ry * HXL + XOFF, *r1 = Hp(b, s1) + ry * HXL + XOFF,
+              *r2 = Hp(b, s2) + ry * HXL + XOFF;
+      if (INT || cen_x) {
+        const int o = INT ? tx : cxo + tx;
+        e0 = sx * csum_t(r0 + o, 1);
+        e1 = sx * csum_t(r1 + o, 1);
+        e2 = sx * csum_t(r2 + o, 1);
+      } else {
+        const R *c = cxs + tx * 11;
+        const int o = cxb[tx];
+        e0 = e1 = e2 = R(0);
 #pragma unroll
-      for (int m = 0; m < 11; ++m) sum += r[m] * c[m];
-      return sx * sum;
+        for (int m = 0; m < 11; ++m) {
+          const R cm = c[m];
+          e0 += r0[o + m] * cm;
+          e1 += r1[o + m] * cm;
+          e2 += r2[o + m] * cm;
+        }
+        e0 *= sx;
+        e1 *= sx;
+        e2 *= sx;
+      }
     };
-    auto DY = [&](int slot) {
-      const R *colp = Hp(b, slot) + rx + XOFF;
-      if (INT) return sy * csum_t(colp + ty * HXL, HXL);
-      if (cen_y) return sy * csum_t(colp + (cyo + ty) * HXL, HXL);
-      const R *r = colp + cyb[ty] * HXL, *c = cys + ty * 11;
-      R sum = R(0);
+    auto DY = [&](int s0, int s1, int s2, R &e0, R &e1, R &e2) {
+      const R *r0 = Hp(b, s0) + rx + XOFF, *r1 = Hp(b, s1) + rx + XOFF,
+              *r2 = Hp(b, s2) + rx + XOFF;
+      if (INT || cen_y) {  // a warp is a row of the tile: no divergence
+        const int o = (ry - 5) * HXL;
+        e0 = sy * csum_t(r0 + o, HXL);
+        e1 = sy * csum_t(r1 + o, HXL);
+        e2 = sy * csum_t(r2 + o, HXL);
+      } else {
+        const R *c = cys + ty * 11;
+        const int o = cyb[ty] * HXL;
+        e0 = e1 = e2 = R(0);
 #pragma unroll
-      for (int m = 0; m < 11; ++m) sum += r[m * HXL] * c[m];
-      return sy * sum;
+        for (int m = 0; m < 11; ++m) {
+          const R cm = c[m];
+          e0 += r0[o + m * HXL] * cm;
+          e1 += r1[o + m * HXL] * cm;
+          e2 += r2[o + m * HXL] * cm;
+        }
+        e0 *= sy;
+        e1 *= sy;
+        e2 *= sy;
+      }
     };
-    const bool zpml = S.zb.on && (k < S.zb.np || k >= nz - S.zt.np);
-    const bool xpml = !INT && S.xb.on && act && (i < S.xb.np || i >= nx - S.xt.np);
-    const bool ypml = !INT && S.yb.on && act && (j < S.yb.np || j >= ny - S.yt.np);
     auto pz = [&](int s0, int s1, int s2, R &da, R &db, R &dc) {
       const bool bot = k < S.zb.np;
       const FaceT<R> &F = bot ? S.zb : S.zt;
@@ -819,18 +865,10 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       cpml3_t<R, MODE>(F, (long long)kl * NXY + col, kl, s0, s1, s2, beta, dt, da, db, dc);
     };
     auto px = [&](int s0, int s1, int s2, R &da, R &db, R &dc) {
-      const bool bot = i < S.xb.np;
-      const FaceT<R> &F = bot ? S.xb : S.xt;
-      const int il = bot ? i : i - (nx - S.xt.np);
-      cpml3_t<R, MODE>(F, il + (long long)F.np * (j + (long long)ny * k), il, s0, s1, s2, beta,
-                     dt, da, db, dc);
+      cpml3_t<R, MODE>(xbot ? S.xb : S.xt, face_x(k), 0, s0, s1, s2, beta, dt, da, db, dc);
     };
     auto py = [&](int s0, int s1, int s2, R &da, R &db, R &dc) {
-      const bool bot = j < S.yb.np;
-      const FaceT<R> &F = bot ? S.yb : S.yt;
-      const int jl = bot ? j : j - (ny - S.yt.np);
-      cpml3_t<R, MODE>(F, i + (long long)nx * (jl + (long long)F.np * k), jl, s0, s1, s2, beta,
-                     dt, da, db, dc);
+      cpml3_t<R, MODE>(ybot ? S.yb : S.yt, face_y(k), 0, s0, s1, s2, beta, dt, da, db, dc);
     };
     auto Hv = [&](int slot) { return Hp(b, slot)[own]; };
     const R iv = IS(1, k);  // velocity (and flux) scale of this layer
@@ -838,8 +876,10 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
     if (act) {
       const R ip = IS(4, k), ib = IS(5, k);
       if (role == 0) {
-        d0 = ip * DX(3); d5 = ib * DX(6); d7 = ib * DX(5);
-        d1 = ip * DY(3); d4 = ib * DY(6); d8 = ib * DY(4);
+        DX(3, 6, 5, d0, d5, d7);
+        DY(3, 6, 4, d1, d4, d8);
+        d0 *= ip; d5 *= ib; d7 *= ib;
+        d1 *= ip; d4 *= ib; d8 *= ib;
         d2 = DZ(0); d6 = DZ(1); d3 = DZ(2);
         if (zpml) pz(1, 2, 3, d2, d6, d3);
         if (xpml) px(1, 3, 2, d0, d5, d7);
@@ -849,8 +889,10 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
         d5 = -d5 + d6;
         d7 = d7 - d8;
       } else {
-        d0 = iv * DX(0); d2 = iv * DX(9); d3 = iv * DX(8);
-        d1 = iv * DY(1); d4 = iv * DY(9); d5 = iv * DY(7);
+        DX(0, 9, 8, d0, d2, d3);
+        DY(1, 9, 7, d1, d4, d5);
+        d0 *= iv; d2 *= iv; d3 *= iv;
+        d1 *= iv; d4 *= iv; d5 *= iv;
         d6 = DZ(0); d7 = DZ(1); d8 = DZ(2);
         if (zpml) pz(4, 5, 0, d7, d6, d8);
         if (xpml) px(0, 4, 5, d0, d2, d3);
@@ -872,7 +914,8 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       const R red = O(b, O_BG + B_RED);
       const R sg = sponge_at(k) ? O(b, O_BG + B_SPONGE) : R(0);
       if (role == 0) {
-        own_loads();
+        const R gk = __ldg(gcol + k);
+        const R frc = S.frc.kind != SPARC_SRC_NONE ? forcing_t(S, Tp, i, j, k) : R(0);
         const R ib = IS(5, k);
         const R cbx = d4, cby = d5, cbz = d7;
         const R c1 = cby * oz - cbz * oy, c2 = ox * cbz - cbx * oz, c3 = cbx * oy - cby * ox;
@@ -927,7 +970,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
           }
           so[l * N + id] = an;
         }
-        if (MODE == F_LAST) VSQ[cid] = vsq;
+        if (MODE == F_LAST) VSQ(b) = vsq;
       } else {
         const R p = Hv(3) * IS(4, k);
         const R div = d0;
@@ -968,7 +1011,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
     if (MODE == F_LAST) {
       bar_pair_t(1 + ty);
       if (act && role == 1) {
-        const double m = ((double)O(b, O_BG + B_RHO0) + an_rho) * VSQ[cid] / 2.0;
+        const double m = ((double)O(b, O_BG + B_RHO0) + an_rho) * VSQ(b) / 2.0;
         ke += m * m;
       }
     }

@@ -236,12 +236,12 @@ int encode_tensor_maps(Handle *h) {
 // chunk) from a device counter until the list is done.  The edge/CPML
 // tiles' items come first (they are the slower ones, so the last items to
 // start are short), each list chunk-major so that neighbouring tiles of a
-// chunk run together; interior tiles take the branch-free body with TMA
-// halo planes, the others the general body.  The diagnostics partials are
+// chunk run together; interior tiles take the branch-free body, the others
+// the general one, both with TMA halo planes (TH; not where halos wrap).  The diagnostics partials are
 // per work item (the last stage reduces each item in the CTA and the item
 // that finishes last sums them in item order), so the norm does not depend
 // on which CTA took which item.
-template <int MODE, bool TMA>
+template <int MODE, bool TMA, bool TH>
 __global__ void __launch_bounds__(mg::NT, 1)
     k_mhd64p(const SimDev S, const __grid_constant__ TmaSet T, const double *__restrict__ a,
              const double *__restrict__ tin, double *__restrict__ so, double beta,
@@ -286,10 +286,10 @@ __global__ void __launch_bounds__(mg::NT, 1)
     // thread 0 takes the next item
     double ke = 0.0, mr = 1e300, mp = 1e300;
     if (in)
-      ok = mhd_body<double, MODE, TMA, true, true>(S, &T, smem, a, tin, so, beta, bnext, x0, y0,
+      ok = mhd_body<double, MODE, TMA, true, TMA, true>(S, &T, smem, a, tin, so, beta, bnext, x0, y0,
                                                    k0, k1, mt, ma, ke, mr, mp, tw);
     else
-      ok = mhd_body<double, MODE, TMA, false, true>(S, &T, smem, a, tin, so, beta, bnext, x0,
+      ok = mhd_body<double, MODE, TMA, false, TH, true>(S, &T, smem, a, tin, so, beta, bnext, x0,
                                                     y0, k0, k1, mt, ma, ke, mr, mp, tw);
     if (!ok) break;
     if (MODE == F_LAST) diag_reduce_t(S, ke, mr, mp, w, total);
@@ -345,8 +345,10 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
   const double bnext = stage < 5 ? h->betas[stage] : h->deltat;
   const int mode = stage == 1 ? FIRST : (stage == 5 ? LAST : MID);
   const bool tma = h->tma && h->allow_tma64;
-  const size_t sm = std::max(MhdBuf<double>::SMEM_GEN,
-                             tma ? MhdBuf<double, true>::SMEM : MhdBuf<double>::SMEM_GEN);
+  // halo boxes for the edge tiles too, except where their halos wrap
+  const bool th = tma && !h->periodic;
+  const size_t sm = tma ? MhdBuf<double, true>::SMEM_GEN : MhdBuf<double>::SMEM_GEN;
+  static_assert(MhdBuf<double, true>::SMEM_GEN + 1024 <= 227 * 1024, "shared memory of an SM");
   int mt = -1, ma = -1;
   for (int b = 0; b < 3; ++b) {
     if (h->buf[b] == tin) mt = b;
@@ -364,20 +366,25 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
   const int grid = (int)std::min<long long>(h->pgrid, total);
   unsigned *ctr = h->d_wctr64 + (stage - 1);
   const dim3 blk(mg::TX, mg::TY, 2);
-#define MP64(M, U)                                                                           \
+#define MP64(M, U, H)                                                                        \
   do {                                                                                       \
-    cudaFuncSetAttribute(k_mhd64p<M, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-    k_mhd64p<M, U><<<grid, blk, sm, s>>>(S, T, a, tin, so, beta, bnext, h->zchunk, mt, ma, h->gix0,   \
+    cudaFuncSetAttribute(k_mhd64p<M, U, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
+                         (int)sm);                                                           \
+    k_mhd64p<M, U, H><<<grid, blk, sm, s>>>(S, T, a, tin, so, beta, bnext, h->zchunk, mt, ma, h->gix0,   \
                                         h->giy0, h->gnix, nint, h->ngen, h->d_gen, ctr);     \
   } while (0)
-  if (tma) {
-    if (mode == FIRST) MP64(F_FIRST, true);
-    else if (mode == MID) MP64(F_MID, true);
-    else MP64(F_LAST, true);
+  if (th) {
+    if (mode == FIRST) MP64(F_FIRST, true, true);
+    else if (mode == MID) MP64(F_MID, true, true);
+    else MP64(F_LAST, true, true);
+  } else if (tma) {
+    if (mode == FIRST) MP64(F_FIRST, true, false);
+    else if (mode == MID) MP64(F_MID, true, false);
+    else MP64(F_LAST, true, false);
   } else {
-    if (mode == FIRST) MP64(F_FIRST, false);
-    else if (mode == MID) MP64(F_MID, false);
-    else MP64(F_LAST, false);
+    if (mode == FIRST) MP64(F_FIRST, false, false);
+    else if (mode == MID) MP64(F_MID, false, false);
+    else MP64(F_LAST, false, false);
   }
 #undef MP64
   return SPARC_OK;

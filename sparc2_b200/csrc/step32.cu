@@ -110,7 +110,7 @@ using MB = MhdBuf<float, false>;
 // with the branch-free body; INT = false covers the whole grid and returns at
 // once on interior tiles.  Each kernel is compiled with one body only, so
 // neither pays the other's registers.
-template <int MODE, bool TMA, bool INT>
+template <int MODE, bool TMA, bool INT, bool TH>
 __global__ void __launch_bounds__(t32::NT, 1)
     k_mhd32(const Sim32 S, const __grid_constant__ TmaSet T,
             const float *__restrict__ a, const float *__restrict__ tin,
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(t32::NT, 1)
   }
   double ke = 0.0, mr = 1e300, mp = 1e300;
   const int k0 = blockIdx.z * zchunk;
-  if (!mhd_body<float, MODE, TMA, INT>(S, &T, smem, a, tin, so, beta, bnext, x0, y0, k0,
+  if (!mhd_body<float, MODE, TMA, INT, TH>(S, &T, smem, a, tin, so, beta, bnext, x0, y0, k0,
                                        min(S.nz, k0 + zchunk), mt, ma, ke, mr, mp))
     return;
   if (MODE == F_LAST)
@@ -397,9 +397,9 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
     }
     if (mt < 0 || ma < 0) return SPARC_ERR_INVALID;
     TmaSet T;
-    std::memset(&T, 0, sizeof(T));  // [18..23]: the plain form's halo maps
+    std::memset(&T, 0, sizeof(T));
     if (h->tma32)
-      for (int n = 0; n < 18; ++n) T.m[n] = h->tmaps32[n];
+      for (int n = 0; n < 24; ++n) T.m[n] = h->tmaps32[n];
     dim3 blk(TX, TY, 2);
     dim3 grd((h->nx + TX - 1) / TX, (h->ny + TYT - 1) / TYT, (h->nz + h->zchunk - 1) / h->zchunk);
     // interior tile rectangle (see mhd_interior), in tile units
@@ -411,36 +411,42 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
     const int iy0 = (ym + TYT - 1) / TYT, iy1 = (h->ny - yM - TYT) / TYT + 1;
     const bool has_int = h->nx - xM - TX >= 0 && h->ny - yM - TYT >= 0 && ix1 > ix0 && iy1 > iy0;
     dim3 gint(has_int ? ix1 - ix0 : 1, has_int ? iy1 - iy0 : 1, grd.z);
-    const int smz = (int)MB::smem_bytes(h->zchunk);
-    // the interior kernel's layout holds 48-wide halo rows with TMA own points
-    const int smi = h->tma32 ? (int)MhdBuf<float, false, true>::smem_bytes(h->zchunk) : smz;
-#define ML32(M, U)                                                                          \
+    const int smi = (int)(h->tma32 ? MhdBuf<float, true>::smem_bytes(h->zchunk)
+                                   : MB::smem_bytes(h->zchunk));
+    // halo boxes for the edge tiles too, except where their halos wrap
+    const bool th = h->tma32 && !h->periodic;
+    const int smz = th ? smi : (int)MB::smem_bytes(h->zchunk);
+#define ML32(M, U, H)                                                                       \
   do {                                                                                      \
-    cudaFuncSetAttribute(k_mhd32<M, U, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi); \
-    cudaFuncSetAttribute(k_mhd32<M, U, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smz); \
+    cudaFuncSetAttribute(k_mhd32<M, U, true, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi); \
+    cudaFuncSetAttribute(k_mhd32<M, U, false, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, smz); \
     if (has_int) {                                                                          \
       cudaEventRecord(h->ev_fork, s);                                                       \
       cudaStreamWaitEvent(h->aux, h->ev_fork, 0);                                           \
-      k_mhd32<M, U, false><<<grd, blk, smz, h->aux>>>(S, T, a, tin, so, beta, bnext,       \
+      k_mhd32<M, U, false, H><<<grd, blk, smz, h->aux>>>(S, T, a, tin, so, beta, bnext,    \
                                                        h->zchunk, mt, ma, 0, 0, gx, gy);    \
       cudaEventRecord(h->ev_join, h->aux);                                                  \
-      k_mhd32<M, U, true><<<gint, blk, smi, s>>>(S, T, a, tin, so, beta, bnext, h->zchunk, \
-                                                  mt, ma, ix0, iy0, gx, gy);                \
+      k_mhd32<M, U, true, U><<<gint, blk, smi, s>>>(S, T, a, tin, so, beta, bnext,         \
+                                                  h->zchunk, mt, ma, ix0, iy0, gx, gy);     \
       cudaStreamWaitEvent(s, h->ev_join, 0);                                                \
     } else {                                                                                \
-      k_mhd32<M, U, false><<<grd, blk, smz, s>>>(S, T, a, tin, so, beta, bnext, h->zchunk, \
-                                                  mt, ma, 0, 0, gx, gy);                    \
+      k_mhd32<M, U, false, H><<<grd, blk, smz, s>>>(S, T, a, tin, so, beta, bnext,         \
+                                                  h->zchunk, mt, ma, 0, 0, gx, gy);         \
     }                                                                                       \
   } while (0)
     if (has_int) ++h->launches;  // the interior launch (counted below: the other)
-    if (h->tma32) {
-      if (mode == F_FIRST) ML32(F_FIRST, true);
-      else if (mode == F_MID) ML32(F_MID, true);
-      else ML32(F_LAST, true);
+    if (th) {
+      if (mode == F_FIRST) ML32(F_FIRST, true, true);
+      else if (mode == F_MID) ML32(F_MID, true, true);
+      else ML32(F_LAST, true, true);
+    } else if (h->tma32) {
+      if (mode == F_FIRST) ML32(F_FIRST, true, false);
+      else if (mode == F_MID) ML32(F_MID, true, false);
+      else ML32(F_LAST, true, false);
     } else {
-      if (mode == F_FIRST) ML32(F_FIRST, false);
-      else if (mode == F_MID) ML32(F_MID, false);
-      else ML32(F_LAST, false);
+      if (mode == F_FIRST) ML32(F_FIRST, false, false);
+      else if (mode == F_MID) ML32(F_MID, false, false);
+      else ML32(F_LAST, false, false);
     }
 #undef ML32
   } else {
@@ -466,10 +472,11 @@ int encode_tensor_maps32(Handle *h) {
                           const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                           const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                           CUtensorMapL2promotion, CUtensorMapFloatOOBfill))fn;
-  auto one = [&](CUtensorMap *m, const float *base, unsigned long long depth) {
+  auto one = [&](CUtensorMap *m, const float *base, unsigned long long depth, int bx = 32,
+                 int by = t32::TYT) {
     cuuint64_t dims[3] = {(cuuint64_t)h->nx, (cuuint64_t)h->ny, (cuuint64_t)depth};
     cuuint64_t strides[2] = {(cuuint64_t)h->nx * 4, (cuuint64_t)h->nx * h->ny * 4};
-    cuuint32_t box[3] = {32, (cuuint32_t)t32::TYT, 1};
+    cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
     cuuint32_t es[3] = {1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)base, dims, strides, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -483,6 +490,12 @@ int encode_tensor_maps32(Handle *h) {
                          FB_GPX, FB_GPY, FB_GPZ, FB_RHOINV, FB_CBX, FB_CBY, FB_CBZ, FB_P0};
   for (int n = 0; n < 15; ++n)
     ok = ok && h->f_bg[order[n]] && one(&h->tmaps32[3 + n], h->f_bg[order[n]], h->nz);
+  constexpr int HXL = MhdBuf<float, true>::HXL;
+  for (int b = 0; b < 3; ++b)
+    ok = ok && one(&h->tmaps32[18 + b], h->fbuf[b], (unsigned long long)h->nz * h->V, HXL, mg::HY);
+  const int b0[3] = {FB_BOX, FB_BOY, FB_BOZ};
+  for (int n = 0; n < 3; ++n)
+    ok = ok && h->f_bg[b0[n]] && one(&h->tmaps32[21 + n], h->f_bg[b0[n]], h->nz, HXL, mg::HY);
   h->tma32 = ok;
   return SPARC_OK;
 }
@@ -580,7 +593,6 @@ template <int MODE, int PART>
 __global__ void __launch_bounds__(BT, 1)
     k_batch_stage(Slot32 *__restrict__ slots, const int4 *__restrict__ items,
                   const int *__restrict__ counts, unsigned *wctr, int stage) {
-  using MB = t32::MB;
   extern __shared__ __align__(1024) float smem_raw32[];
   __shared__ __align__(16) unsigned long long sS_raw[(sizeof(Sim32) + 7) / 8];
   __shared__ int s_w;
@@ -615,10 +627,10 @@ __global__ void __launch_bounds__(BT, 1)
     const int x0 = it.y, y0 = it.z, k0 = it.w & 0xffff, k1 = it.w >> 16;
     double ke = 0.0, mr = 1e300, mp = 1e300;
     if (PART == 0 || (PART == 2 && w < counts[3]))
-      mhd_body<float, MODE, false, true>(sS, nullptr, smem, a, tin, so, beta, bnext, x0, y0,
+      mhd_body<float, MODE, false, true, false>(sS, nullptr, smem, a, tin, so, beta, bnext, x0, y0,
                                          k0, k1, 0, 0, ke, mr, mp);
     else if (sS.magnetic)
-      mhd_body<float, MODE, false, false>(sS, nullptr, smem, a, tin, so, beta, bnext, x0, y0,
+      mhd_body<float, MODE, false, false, false>(sS, nullptr, smem, a, tin, so, beta, bnext, x0, y0,
                                           k0, k1, 0, 0, ke, mr, mp);
     else if (sS.bg1d)
       quiet_body<float, 16, MODE, true, MODE == F_LAST ? 2 : 3>(sS, smem, a, tin, so, beta, bnext, x0, y0, k0, k1,
