@@ -163,6 +163,13 @@ enum {
 // memory, and longer chunks let the blocks of neighbouring tiles drift apart
 constexpr int QUIET_ZMAX = 32;
 
+// MHD: the 3-D background arrays of a handle lie one after another in one
+// allocation, in this order, so that one tensor copy brings several
+enum {
+  PK_RED, PK_RHO0, PK_GRX, PK_GRY, PK_GRZ, PK_C2R, PK_GPX, PK_GPY, PK_GPZ, PK_RHOINV, PK_CBX,
+  PK_CBY, PK_CBZ, PK_SPONGE, PK_P0, PK_BOX, PK_BOY, PK_BOZ, PK_COUNT
+};
+
 struct Handle {
   sparc_params P{};
   int device = 0;
@@ -235,10 +242,11 @@ struct Handle {
   float *f_f2d = nullptr, *f_sdep = nullptr;
   int nblocks = 1;
 
-  // TMA tensor maps (32x8x1 boxes) of the MHD own-point arrays: [0..2] the
-  // state buffers (nx, ny, nz*V), [3..17] the background arrays per layer
+  // MHD: the packed background (FP64 or FP32) and the tensor maps of the
+  // stage kernels (as TmaSet of mhd_body.cuh)
+  void *bg_pack = nullptr;
   bool tma = false;
-  CUtensorMap tmaps_ty[24];
+  CUtensorMap tmaps[12];
   // FILTER_VARS xy pass (non-periodic FP64 grids, nx even): the state
   // buffers in 44x44x1 boxes
   bool ftma = false;
@@ -279,10 +287,8 @@ struct Handle {
   float *f_fx = nullptr, *f_fy = nullptr, *f_fz = nullptr;
   float *f_psr = nullptr, *f_px = nullptr, *f_py = nullptr;
   float *f_sd = nullptr, *f_ssb = nullptr;
-  bool tma32 = false;
   bool allow_tma32 = true;   // FP32 MHD own-point loads by TMA (nx % 4 == 0)
   bool allow_tma64 = true;   // FP64 MHD own-point loads by TMA (nx even)
-  CUtensorMap tmaps32[24];  // as TmaSet (mhd_body.cuh)
 
   // member of a batch (sparc_batch_add): the batch owns the buffer roles,
   // the iteration and the stream order until sparc_batch_remove
@@ -324,6 +330,7 @@ int launch_random_forcing(Handle *h, cudaStream_t s);
 int launch_filter_event(Handle *h, bool xy, const double *in, double *out, cudaStream_t s);
 int stage_geometry(Handle *h);
 int encode_tensor_maps(Handle *h);
+bool encode_stage_maps(Handle *h, int hxl);
 
 // step32.cu (precision form)
 int step32_constants();
@@ -336,7 +343,6 @@ int launch_batch_step(const BatchLaunch &B, cudaStream_t s, int *nkernels);
 size_t batch_stage_smem();
 int launch_filter_event32(Handle *h, bool xy, const float *in, const float *carry, float *out,
                           cudaStream_t s);
-int encode_tensor_maps32(Handle *h);
 int setup32(Handle *h);
 int damping_setup(Handle *h);
 int mhd64_plan(Handle *h);

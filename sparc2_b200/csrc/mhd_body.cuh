@@ -34,14 +34,18 @@ constexpr int NH = 10, NO = 24;
 constexpr long long WAIT_LIMIT = kMbarWaitLimit;
 // own-point slots: stage rho, a[0..7], 14 background arrays, p0
 constexpr int O_RHO = 0, O_A = 1, O_BG = 9, O_P0 = 23;
-enum { B_RED, B_SPONGE, B_RHO0, B_GRX, B_GRY, B_GRZ, B_C2R, B_GPX, B_GPY,
-       B_GPZ, B_RHOINV, B_CBX, B_CBY, B_CBZ };
+// (the order of the packed background arrays, internal.h)
+enum { B_RED = PK_RED, B_RHO0 = PK_RHO0, B_GRX = PK_GRX, B_GRY = PK_GRY, B_GRZ = PK_GRZ,
+       B_C2R = PK_C2R, B_GPX = PK_GPX, B_GPY = PK_GPY, B_GPZ = PK_GPZ, B_RHOINV = PK_RHOINV,
+       B_CBX = PK_CBX, B_CBY = PK_CBY, B_CBZ = PK_CBZ, B_SPONGE = PK_SPONGE };
+static_assert(O_BG + PK_P0 == O_P0, "own-point slots in the packed order");
 }  // namespace mg
 
 // shared-memory buffers of one layer (in R words, 128-byte multiple) and the
 // dynamic size.  TH: the halo planes arrive as TMA boxes, whose rows start at
 // a 16-byte aligned column (x0 - 6 in FP64, 44 wide; x0 - 8 in FP32, 48 wide),
-// each plane 128-byte aligned; otherwise 42 x 18 copied by cp.async.  The
+// seven state planes as one box and three B0 planes as another; otherwise
+// 42 x 18 copied by cp.async.  The
 // precision form keeps |v_new|^2 of the last stage (FP64) after the buffers;
 // the plain form has it in the slot of a value already used.
 template <class R, bool TH = false>
@@ -49,8 +53,10 @@ struct MhdBuf {
   static constexpr int ALIGN = 128 / (int)sizeof(R);
   static constexpr int HXL = TH ? (sizeof(R) == 8 ? 44 : 48) : mg::HX;
   static constexpr int XOFF = TH ? (sizeof(R) == 8 ? 1 : 3) : 0;
-  static constexpr int HSL = TH ? (HXL * mg::HY + ALIGN - 1) / ALIGN * ALIGN : mg::HS;
-  static constexpr int BUF = ((mg::NO * mg::NC + mg::NH * HSL) + ALIGN - 1) / ALIGN * ALIGN;
+  static constexpr int HSL = HXL * mg::HY;  // a plane
+  // the three B0 planes start at HB (their own box: 128-byte aligned)
+  static constexpr int HB = TH ? (7 * HSL + ALIGN - 1) / ALIGN * ALIGN : 7 * HSL;
+  static constexpr int BUF = (mg::NO * mg::NC + HB + 3 * HSL + ALIGN - 1) / ALIGN * ALIGN;
   static constexpr int XCH = sizeof(R) == 4 ? 2 * mg::NC : 0;
   static constexpr size_t SMEM = (2 * (size_t)BUF + XCH) * sizeof(R) + 128;
   // plain form, general tiles: the per-lane and per-row coefficient tables
@@ -65,11 +71,13 @@ struct MhdBuf {
   }
 };
 
-// tensor maps: [0..2] the state buffers (nx, ny, nz*V) and [3..17] the
-// background arrays in 32x8x1 boxes (own points); [18..20] the state buffers
-// and [21..23] B0 x, y, z in halo boxes (44x18x1 FP64, 48x18x1 FP32)
+// tensor maps, all of 4-D views: the state buffers (nx, ny, nz, V) in boxes
+// of one field's 32 x 8 own points [0..2], of all fields' [3..5] and of seven
+// fields' halo planes [6..8]; the packed background (nx, ny, nz, 18) in boxes
+// of 13 arrays' own points [9], of one's [10] and of the three B0 halo
+// planes [11]
 struct TmaSet {
-  CUtensorMap m[24];
+  CUtensorMap m[12];
 };
 
 template <class R>
@@ -376,7 +384,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   using namespace mg;
   static_assert(TMA || !TH, "halo boxes come with the own-point boxes");
   using MB = MhdBuf<R, TH>;
-  constexpr int BUF = MB::BUF, HXL = MB::HXL, XOFF = MB::XOFF, HSL = MB::HSL;
+  constexpr int BUF = MB::BUF, HXL = MB::HXL, XOFF = MB::XOFF, HSL = MB::HSL, HB = MB::HB;
   constexpr bool SCALED = sizeof(R) == 4;
   __shared__ unsigned long long bar[2];
   const int tx = threadIdx.x, ty = threadIdx.y, role = threadIdx.z;
@@ -462,7 +470,9 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   }
   __syncthreads();
   auto O = [&](int b, int slot) -> R { return smem[b * BUF + slot * NC + cid]; };
-  auto Hp = [&](int b, int slot) -> R * { return smem + b * BUF + NO * NC + slot * HSL; };
+  auto Hp = [&](int b, int slot) -> R * {
+    return smem + b * BUF + NO * NC + (slot < 7 ? slot * HSL : HB + (slot - 7) * HSL);
+  };
   // |v_new|^2 of the last stage (role 0 writes, role 1 reads after a barrier);
   // plain form: in the slot of a[1], which its writer has read
   auto VSQ = [&](int b) -> double & {
@@ -513,10 +523,6 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   auto sponge_at = [&](int k) -> bool {
     return !S.sponge_slabs || slab_xy || (S.zb.on && (k < S.zb.np || k >= nz - S.zt.np));
   };
-  auto skip_own = [&](int c, int k) -> bool {
-    return (MODE == F_FIRST && c >= O_A && c < O_BG) || (MODE != F_LAST && c == O_P0) ||
-           (c == O_BG + B_SPONGE && !sponge_at(k));
-  };
   auto own_bytes = [&](int k) -> unsigned {
     return ((MODE == F_FIRST ? 15u : (MODE == F_MID ? 23u : 24u)) -
             (sponge_at(k) ? 0u : 1u)) *
@@ -530,18 +536,18 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       const int id = kb + ho0;
 #pragma unroll
       for (int sl = 0; sl < 7; ++sl) cp_r(h + sl * HSL, tin + (sl + 1) * N + id);
-      cp_r(h + 7 * HSL, S.box + id);
-      cp_r(h + 8 * HSL, S.boy + id);
-      cp_r(h + 9 * HSL, S.boz + id);
+      cp_r(h + HB, S.box + id);
+      cp_r(h + HB + HSL, S.boy + id);
+      cp_r(h + HB + 2 * HSL, S.boz + id);
     }
     if (!TH && hs1 >= 0) {
       R *h = Hp(b, 0) + hs1;
       const int id = kb + ho1;
 #pragma unroll
       for (int sl = 0; sl < 7; ++sl) cp_r(h + sl * HSL, tin + (sl + 1) * N + id);
-      cp_r(h + 7 * HSL, S.box + id);
-      cp_r(h + 8 * HSL, S.boy + id);
-      cp_r(h + 9 * HSL, S.boz + id);
+      cp_r(h + HB, S.box + id);
+      cp_r(h + HB + HSL, S.boy + id);
+      cp_r(h + HB + 2 * HSL, S.boz + id);
     }
     if (!TMA && act) {
       R *ob = smem + b * BUF + cid;
@@ -552,8 +558,8 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
 #pragma unroll
           for (int l = 0; l < 8; ++l) cp_r(ob + (O_A + l) * NC, a + l * N + id);
       } else {
-        const R *bg[14] = {S.red, S.sponge, S.rho0, S.grx, S.gry, S.grz,
-                               S.c2rho0, S.gpx, S.gpy, S.gpz, S.rhoinv, S.cbx, S.cby, S.cbz};
+        const R *bg[14] = {S.red, S.rho0, S.grx, S.gry, S.grz, S.c2rho0, S.gpx,
+                           S.gpy, S.gpz, S.rhoinv, S.cbx, S.cby, S.cbz, S.sponge};
         const bool spg = sponge_at(k);
 #pragma unroll
         for (int n = 0; n < 14; ++n)
@@ -563,39 +569,30 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       }
     }
     cp_commit_t();
-    // TMA copies of the layer, spread over all warps (lane l of warp w issues
-    // copy 16 l + w; a warp that issued all of them held up every layer: FP64
-    // 256x256x300 12.58 -> 12.24 ms per iteration): copy c < 24 is own slot c
-    // (stage rho, a[0..7], 14 background arrays, p0); with TH, copy 24 + s is
-    // halo plane s (state fields 1..7, then B0 x, y, z).  Copies may complete
-    // before thread 0's expect: the phase ends with its arrival at the
-    // earliest.
-    if (TMA && tx < (TH ? 3 : 2)) {
-      if (tid == 0) mbar_tx_t(&bar[b], own_bytes(k));
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // TMA copies of the layer: five to seven boxes of several fields each,
+    // one per warp.  (One box per field, 34 a layer, cost the issuing warps a
+    // fifth of an interior layer's time: the copy engine takes them one after
+    // another.)  Copies may complete before thread 0's expect: the phase ends
+    // with its arrival at the earliest.
+    if (TMA && tx == 0 && (tid >> 5) < 6) {
+      const int w = tid >> 5;
       R *ob = smem + b * BUF;
-      const int c = tx * 16 + (tid >> 5);
-      if (c < (TH ? NO + NH : NO) && !skip_own(c, k)) {
-        int map = mt, xx = x0, yy = y0, z = k;
-        R *dst = ob + c * NC;
-        if (c >= O_A && c < O_BG) {
-          map = ma;
-          z = (c - O_A) * nz + k;
-        } else if (c >= O_BG && c <= O_P0) {
-          map = 3 + (c - O_BG);
-        } else if (c >= NO) {
-          const int sl = c - NO;
-          dst = Hp(b, sl);
-          xx = xo - XOFF;
-          yy = yo;
-          if (sl < 7) {
-            map = 18 + mt;
-            z = (sl + 1) * nz + k;
-          } else {
-            map = 21 + (sl - 7);
-          }
-        }
-        tma3d_t(dst, &T->m[map], xx, yy, z, &bar[b]);
+      unsigned long long *br = &bar[b];
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      if (w == 0) {
+        mbar_tx_t(br, own_bytes(k));
+        tma4d_t(ob + O_RHO * NC, &T->m[mt], x0, y0, k, 0, br);
+      } else if (w == 1) {
+        if (MODE != F_FIRST) tma4d_t(ob + O_A * NC, &T->m[3 + ma], x0, y0, k, 0, br);
+      } else if (w == 2) {
+        tma4d_t(ob + O_BG * NC, &T->m[9], x0, y0, k, 0, br);
+      } else if (w == 3) {
+        if (TH) tma4d_t(Hp(b, 0), &T->m[6 + mt], xo - XOFF, yo, k, 1, br);
+      } else if (w == 4) {
+        if (TH) tma4d_t(Hp(b, 7), &T->m[11], xo - XOFF, yo, k, PK_BOX, br);
+      } else {
+        if (sponge_at(k)) tma4d_t(ob + (O_BG + B_SPONGE) * NC, &T->m[10], x0, y0, k, PK_SPONGE, br);
+        if (MODE == F_LAST) tma4d_t(ob + O_P0 * NC, &T->m[10], x0, y0, k, PK_P0, br);
       }
     }
   };
@@ -604,12 +601,12 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   auto flux = [&](int b, int t, R &bx0, R &by0, R &bz0) {
     R *H = Hp(b, 0) + t;
     const R vx_ = H[0], vy_ = H[HSL], vz_ = H[2 * HSL];
-    bx0 = H[7 * HSL];
-    by0 = H[8 * HSL];
-    bz0 = H[9 * HSL];
-    H[7 * HSL] = -vz_ * by0 + vy_ * bz0;
-    H[8 * HSL] = -vx_ * bz0 + vz_ * bx0;
-    H[9 * HSL] = -vy_ * bx0 + vx_ * by0;
+    bx0 = H[HB];
+    by0 = H[HB + HSL];
+    bz0 = H[HB + 2 * HSL];
+    H[HB] = -vz_ * by0 + vy_ * bz0;
+    H[HB + HSL] = -vx_ * bz0 + vz_ * bx0;
+    H[HB + 2 * HSL] = -vy_ * bx0 + vx_ * by0;
   };
   R w0[11], w1[11], w2[11];  // physical values
   // The values a window head of layer kk is made of, and the head: momentum

@@ -357,8 +357,15 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
   if (!h->d_stretch) return SPARC_ERR_NOMEM;
 
   // ------------------------------------------------ 3-D arrays (FP64)
-  double *rho0 = h->rho0 = up(h, nullptr, N);
-  double *p0 = h->p0 = up(h, nullptr, N);
+  // MHD in the plain form: the arrays of the stage kernels in one allocation
+  double *pack = nullptr;
+  if (h->magnetic && !h->fp32) {
+    h->bg_pack = pack = up(h, nullptr, PK_COUNT * N);
+    if (!pack) return SPARC_ERR_NOMEM;
+  }
+  auto bga = [&](int n) -> double * { return pack ? pack + n * N : up(h, nullptr, N); };
+  double *rho0 = h->rho0 = bga(PK_RHO0);
+  double *p0 = h->p0 = bga(PK_P0);
   double *c2 = h->c2 = up(h, nullptr, N);
   double *cs = up(h, nullptr, N);
   if (!rho0 || !p0 || !c2 || !cs) return SPARC_ERR_NOMEM;
@@ -387,9 +394,9 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
   if (!ssb) return SPARC_ERR_NOMEM;
   double *box = nullptr, *boy = nullptr, *boz = nullptr;
   if (h->magnetic) {
-    box = h->box = up(h, nullptr, N);
-    boy = h->boy = up(h, nullptr, N);
-    boz = h->boz = up(h, nullptr, N);
+    box = h->box = bga(PK_BOX);
+    boy = h->boy = bga(PK_BOY);
+    boz = h->boz = bga(PK_BOZ);
     if (!box || !boy || !boz) return SPARC_ERR_NOMEM;
     CK(cudaMemcpyAsync(box, bx0, N * 8, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(boy, by0, N * 8, cudaMemcpyHostToDevice, s));
@@ -446,7 +453,7 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
     std::copy(sx.begin(), sx.end(), all.begin() + nz);
     std::copy(sy.begin(), sy.end(), all.begin() + nz + nx);
     double *d = up(h, all.data(), all.size());
-    double *sponge = h->sponge = up(h, nullptr, N);
+    double *sponge = h->sponge = bga(PK_SPONGE);
     if (!d || !sponge) return SPARC_ERR_NOMEM;
     const bool per = h->periodic;
     each(N, s, [=] __device__(long long n) {
@@ -459,7 +466,7 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
   if (!tmp) return SPARC_ERR_NOMEM;
   if (h->magnetic) {
     // Alfven limiter, initialize.f90:962-991
-    double *red = h->red = up(h, nullptr, N);
+    double *red = h->red = bga(PK_RED);
     double *dcq = up(h, h->cq.data(), nz);
     unsigned long long *dmax = (unsigned long long *)dev_alloc(h, 8 * kVaCand);
     if (!red || !dcq || !dmax) return SPARC_ERR_NOMEM;
@@ -531,9 +538,9 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
     }
     each(N, s, [=] __device__(long long n) { red[n] = T / (T + red[n]); });
     // curl B0, initialize.f90:993-1006
-    double *cbx = h->cbx = up(h, nullptr, N);
-    double *cby = h->cby = up(h, nullptr, N);
-    double *cbz = h->cbz = up(h, nullptr, N);
+    double *cbx = h->cbx = bga(PK_CBX);
+    double *cby = h->cby = bga(PK_CBY);
+    double *cbz = h->cbz = bga(PK_CBZ);
     if (!cbx || !cby || !cbz) return SPARC_ERR_NOMEM;
     int r = 0;
     r |= launch_derivative(h, 0, bc, boy, cbz, s);
@@ -548,10 +555,10 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
     if (r) return SPARC_ERR_CUDA;
   }
   // initialize.f90:1012-1034
-  double *rhoinv = h->rhoinv = up(h, nullptr, N);
-  double *c2rho0 = h->c2rho0 = up(h, nullptr, N);
-  double *grz = h->grz = up(h, nullptr, N);
-  double *gpz = h->gpz = up(h, nullptr, N);
+  double *rhoinv = h->rhoinv = bga(PK_RHOINV);
+  double *c2rho0 = h->c2rho0 = bga(PK_C2R);
+  double *grz = h->grz = bga(PK_GRZ);
+  double *gpz = h->gpz = bga(PK_GPZ);
   if (!rhoinv || !c2rho0 || !grz || !gpz) return SPARC_ERR_NOMEM;
   each(N, s, [=] __device__(long long n) {
     rhoinv[n] = 1.0 / rho0[n];
@@ -714,8 +721,8 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
     each(N, s, [=] __device__(long long n) { sd[n] = per ? 1.0 : 1.0 - sd[n]; });
   }
   if (h->magnetic) {  // initialize.f90:1219-1228
-    h->grx = up(h, nullptr, N); h->gpx = up(h, nullptr, N);
-    h->gry = up(h, nullptr, N); h->gpy = up(h, nullptr, N);
+    h->grx = bga(PK_GRX); h->gpx = bga(PK_GPX);
+    h->gry = bga(PK_GRY); h->gpy = bga(PK_GPY);
     if (!h->grx || !h->gpx || !h->gry || !h->gpy) return SPARC_ERR_NOMEM;
     if (launch_derivative(h, 0, bc, rho0, h->grx, s) ||
         launch_derivative(h, 0, bc, p0, h->gpx, s) ||

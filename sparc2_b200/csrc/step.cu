@@ -153,15 +153,15 @@ static int launch_quiet(Handle *h, const SimDev &S, int stage, const double *a,
 }
 
 int encode_tensor_maps(Handle *h) {
-  h->tma = false;
   h->ftma = false;
   // rows of a multiple of 16 bytes; the filter's tiles read zero outside
   // the grid, so its maps serve non-periodic grids only
   const bool want_f = !h->periodic && !(h->nx & 1);
-  const bool want_m = h->magnetic && !(h->nx & 1);
   h->ztma = false;
   const bool want_z = !(h->nx & 1);
-  if (!want_f && !want_m && !want_z) return SPARC_OK;
+  h->tma = h->magnetic && !(h->nx & 1) && h->allow_tma64 &&
+           encode_stage_maps(h, MhdBuf<double, true>::HXL);
+  if (!want_f && !want_z) return SPARC_OK;
   void *fn = nullptr;
   cudaDriverEntryPointQueryResult q;
   if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) !=
@@ -183,10 +183,6 @@ int encode_tensor_maps(Handle *h) {
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-  };
-  auto one = [&](CUtensorMap *m, const double *base, unsigned long long depth, bool halo = false) {
-    return boxed(m, base, depth, halo ? MhdBuf<double, true>::HXL : mg::TX,
-                 halo ? mg::HY : mg::TY);
   };
   if (want_f) {
     // FILTER_VARS xy pass: the 44 x 44 neighbourhood of a 32 x 32 tile
@@ -215,18 +211,47 @@ int encode_tensor_maps(Handle *h) {
     }
     h->ztma = zok;
   }
-  if (!want_m) return SPARC_OK;
-  bool ok = true;
-  for (int b = 0; b < 3; ++b) ok = ok && one(&h->tmaps_ty[b], h->buf[b], (unsigned long long)h->nz * h->V);
-  const double *bg[15] = {h->red, h->sponge, h->rho0, h->grx, h->gry, h->grz, h->c2rho0,
-                          h->gpx, h->gpy, h->gpz, h->rhoinv, h->cbx, h->cby, h->cbz, h->p0};
-  for (int n = 0; n < 15; ++n) ok = ok && bg[n] && one(&h->tmaps_ty[3 + n], bg[n], h->nz);
-  for (int b = 0; b < 3; ++b)
-    ok = ok && one(&h->tmaps_ty[18 + b], h->buf[b], (unsigned long long)h->nz * h->V, true);
-  const double *b0[3] = {h->box, h->boy, h->boz};
-  for (int n = 0; n < 3; ++n) ok = ok && b0[n] && one(&h->tmaps_ty[21 + n], b0[n], h->nz, true);
-  h->tma = ok;
   return SPARC_OK;
+}
+
+// The tensor maps of the MHD stage kernels, as TmaSet lists them (both
+// precisions: rows of a multiple of 16 bytes; hxl: the columns of a halo
+// box).  False where the driver does not give them; the cp.async kernels
+// serve then.
+bool encode_stage_maps(Handle *h, int hxl) {
+  void *fn = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) !=
+          cudaSuccess || !fn || q != cudaDriverEntryPointSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  auto enc = (CUresult(*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
+                          const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                          const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                          CUtensorMapL2promotion, CUtensorMapFloatOOBfill))fn;
+  const cuuint64_t w = h->fp32 ? 4 : 8, nx = h->nx, ny = h->ny, nz = h->nz;
+  auto one = [&](CUtensorMap *m, void *base, int fields, int bx, int by, int bf) {
+    if (!base) return false;
+    const cuuint64_t dims[4] = {nx, ny, nz, (cuuint64_t)fields};
+    const cuuint64_t strides[3] = {nx * w, nx * ny * w, nx * ny * nz * w};
+    const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, 1, (cuuint32_t)bf};
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    return enc(m, h->fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
+               base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  bool ok = true;
+  for (int b = 0; b < 3; ++b) {
+    void *st = h->fp32 ? (void *)h->fbuf[b] : (void *)h->buf[b];
+    ok = ok && one(&h->tmaps[b], st, h->V, mg::TX, mg::TY, 1) &&
+         one(&h->tmaps[3 + b], st, h->V, mg::TX, mg::TY, 8) &&
+         one(&h->tmaps[6 + b], st, h->V, hxl, mg::HY, 7);
+  }
+  return ok && one(&h->tmaps[9], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 13) &&
+         one(&h->tmaps[10], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 1) &&
+         one(&h->tmaps[11], h->bg_pack, PK_COUNT, hxl, mg::HY, 3);
 }
 
 // ------------------------- MP_MHD_3D, shared-body stage kernel
@@ -344,7 +369,7 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
   const double beta = h->betas[stage - 1];
   const double bnext = stage < 5 ? h->betas[stage] : h->deltat;
   const int mode = stage == 1 ? FIRST : (stage == 5 ? LAST : MID);
-  const bool tma = h->tma && h->allow_tma64;
+  const bool tma = h->tma;
   // halo boxes for the edge tiles too, except where their halos wrap
   const bool th = tma && !h->periodic;
   const size_t sm = tma ? MhdBuf<double, true>::SMEM_GEN : MhdBuf<double>::SMEM_GEN;
@@ -357,7 +382,7 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
   if (mt < 0 || ma < 0 || !h->d_wctr64) return SPARC_ERR_INVALID;
   TmaSet T;
   if (tma)
-    for (int n = 0; n < 24; ++n) T.m[n] = h->tmaps_ty[n];
+    std::memcpy(&T, h->tmaps, sizeof(T));
   else
     std::memset(&T, 0, sizeof(T));
   const int nch = (h->nz + h->zchunk - 1) / h->zchunk;

@@ -397,9 +397,10 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
     }
     if (mt < 0 || ma < 0) return SPARC_ERR_INVALID;
     TmaSet T;
-    std::memset(&T, 0, sizeof(T));
-    if (h->tma32)
-      for (int n = 0; n < 24; ++n) T.m[n] = h->tmaps32[n];
+    if (h->tma)
+      std::memcpy(&T, h->tmaps, sizeof(T));
+    else
+      std::memset(&T, 0, sizeof(T));
     dim3 blk(TX, TY, 2);
     dim3 grd((h->nx + TX - 1) / TX, (h->ny + TYT - 1) / TYT, (h->nz + h->zchunk - 1) / h->zchunk);
     // interior tile rectangle (see mhd_interior), in tile units
@@ -411,10 +412,10 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
     const int iy0 = (ym + TYT - 1) / TYT, iy1 = (h->ny - yM - TYT) / TYT + 1;
     const bool has_int = h->nx - xM - TX >= 0 && h->ny - yM - TYT >= 0 && ix1 > ix0 && iy1 > iy0;
     dim3 gint(has_int ? ix1 - ix0 : 1, has_int ? iy1 - iy0 : 1, grd.z);
-    const int smi = (int)(h->tma32 ? MhdBuf<float, true>::smem_bytes(h->zchunk)
+    const int smi = (int)(h->tma ? MhdBuf<float, true>::smem_bytes(h->zchunk)
                                    : MB::smem_bytes(h->zchunk));
     // halo boxes for the edge tiles too, except where their halos wrap
-    const bool th = h->tma32 && !h->periodic;
+    const bool th = h->tma && !h->periodic;
     const int smz = th ? smi : (int)MB::smem_bytes(h->zchunk);
 #define ML32(M, U, H)                                                                       \
   do {                                                                                      \
@@ -439,7 +440,7 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
       if (mode == F_FIRST) ML32(F_FIRST, true, true);
       else if (mode == F_MID) ML32(F_MID, true, true);
       else ML32(F_LAST, true, true);
-    } else if (h->tma32) {
+    } else if (h->tma) {
       if (mode == F_FIRST) ML32(F_FIRST, true, false);
       else if (mode == F_MID) ML32(F_MID, true, false);
       else ML32(F_LAST, true, false);
@@ -454,50 +455,6 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
   }
   ++h->launches;
   return cudaGetLastError() == cudaSuccess ? SPARC_OK : SPARC_ERR_CUDA;
-}
-
-// FP32 tensor maps (32 x TYT x 1 boxes) of the own-point arrays of the MHD kernel
-// (needs 16-byte row strides: nx a multiple of 4).
-int encode_tensor_maps32(Handle *h) {
-  h->tma32 = false;
-  if (!h->magnetic || (h->nx & 3) || !h->allow_tma32) return SPARC_OK;
-  void *fn = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) !=
-          cudaSuccess || !fn || q != cudaDriverEntryPointSuccess) {
-    cudaGetLastError();
-    return SPARC_OK;
-  }
-  auto enc = (CUresult(*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                          const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                          const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                          CUtensorMapL2promotion, CUtensorMapFloatOOBfill))fn;
-  auto one = [&](CUtensorMap *m, const float *base, unsigned long long depth, int bx = 32,
-                 int by = t32::TYT) {
-    cuuint64_t dims[3] = {(cuuint64_t)h->nx, (cuuint64_t)h->ny, (cuuint64_t)depth};
-    cuuint64_t strides[2] = {(cuuint64_t)h->nx * 4, (cuuint64_t)h->nx * h->ny * 4};
-    cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
-    cuuint32_t es[3] = {1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)base, dims, strides, box, es,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-  };
-  bool ok = true;
-  for (int b = 0; b < 3; ++b)
-    ok = ok && one(&h->tmaps32[b], h->fbuf[b], (unsigned long long)h->nz * h->V);
-  const int order[15] = {FB_RED, FB_SPONGE, FB_RHO0, FB_GRX, FB_GRY, FB_GRZ, FB_C2R,
-                         FB_GPX, FB_GPY, FB_GPZ, FB_RHOINV, FB_CBX, FB_CBY, FB_CBZ, FB_P0};
-  for (int n = 0; n < 15; ++n)
-    ok = ok && h->f_bg[order[n]] && one(&h->tmaps32[3 + n], h->f_bg[order[n]], h->nz);
-  constexpr int HXL = MhdBuf<float, true>::HXL;
-  for (int b = 0; b < 3; ++b)
-    ok = ok && one(&h->tmaps32[18 + b], h->fbuf[b], (unsigned long long)h->nz * h->V, HXL, mg::HY);
-  const int b0[3] = {FB_BOX, FB_BOY, FB_BOZ};
-  for (int n = 0; n < 3; ++n)
-    ok = ok && h->f_bg[b0[n]] && one(&h->tmaps32[21 + n], h->f_bg[b0[n]], h->nz, HXL, mg::HY);
-  h->tma32 = ok;
-  return SPARC_OK;
 }
 
 // ------------------------------------------------------------ batched engine
@@ -941,10 +898,24 @@ int setup32(Handle *h) {
       {FB_CBZ, h->cbz, nullptr},         {FB_GRX, h->grx, nullptr},
       {FB_GRY, h->gry, nullptr},         {FB_GPX, h->gpx, nullptr},
       {FB_GPY, h->gpy, nullptr},         {FB_RED, h->red, nullptr}};
+  // MHD: one allocation in the packed order
+  static const int packed[PK_COUNT] = {FB_RED, FB_RHO0, FB_GRX, FB_GRY, FB_GRZ, FB_C2R,
+                                       FB_GPX, FB_GPY, FB_GPZ, FB_RHOINV, FB_CBX, FB_CBY,
+                                       FB_CBZ, FB_SPONGE, FB_P0, FB_BOX, FB_BOY, FB_BOZ};
+  if (h->magnetic) {
+    float *pack = f_up(h, nullptr, PK_COUNT * N, s);
+    if (!pack) return SPARC_ERR_NOMEM;
+    h->bg_pack = pack;
+    for (int n = 0; n < PK_COUNT; ++n) h->f_bg[packed[n]] = pack + n * N;
+  }
   for (const Src &q : srcs) {
     const bool one = h->bg1d && q.d1;
     const double *src = one ? q.d1 : q.d3;
     if (!src) continue;
+    if (h->f_bg[q.fb]) {
+      if (to_float(src, h->f_bg[q.fb], N, s)) return SPARC_ERR_CUDA;
+      continue;
+    }
     h->f_bg[q.fb] = f_up(h, src, one ? nz : N, s);
     if (!h->f_bg[q.fb]) return SPARC_ERR_NOMEM;
   }
@@ -988,7 +959,9 @@ int setup32(Handle *h) {
     dev_free(h, D.pki);
     D.pa = D.pb = D.pk = D.pki = nullptr;
   }
-  return encode_tensor_maps32(h);
+  h->tma = h->magnetic && !(h->nx & 3) && h->allow_tma32 &&
+           encode_stage_maps(h, MhdBuf<float, true>::HXL);
+  return SPARC_OK;
 }
 
 // FP32 copies of the forcing tables built by sparc_set_source.
