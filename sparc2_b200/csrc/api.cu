@@ -485,6 +485,11 @@ int sparc_create(const sparc_params *p, int device, sparc_handle **out) {
     h->d_iter = (long long *)dev_alloc(h, 8);
     h->d_fail = (long long *)dev_alloc(h, 8);
     h->d_partials = (double *)dev_alloc(h, (size_t)h->partials_blocks * 3 * 8);
+    if (h->magnetic) {  // two parts per 4-layer segment of a 32 x 8 tile
+      const size_t tiles = (size_t)((h->nx + 31) / 32) * ((h->ny + 7) / 8);
+      h->d_kseg = (double *)dev_alloc(h, 2 * tiles * ((h->nz + 3) / 4) * 8);
+      if (!h->d_kseg) r = SPARC_ERR_NOMEM;
+    }
     h->d_diag = (double *)dev_alloc(h, 4 * 8);
     h->d_counter = (unsigned int *)dev_alloc(h, 4);
     if (!h->d_iter || !h->d_fail || !h->d_partials || !h->d_diag || !h->d_counter)

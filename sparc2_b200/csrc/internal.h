@@ -83,6 +83,7 @@ struct SimT {
   long long *iter;             // current driver iteration
   int *err;                    // device error flag (bounded waits)
   double *partials;            // 3 per block of the last stage
+  double *kseg;                // MHD: KE sums of 4-layer tile segments
   unsigned int *counter;
   double *diag;                // ke, min_rho, min_p, iteration(double)
   long long *fail_iter;
@@ -246,7 +247,7 @@ struct Handle {
   // stage kernels (as TmaSet of mhd_body.cuh)
   void *bg_pack = nullptr;
   bool tma = false;
-  CUtensorMap tmaps[12];
+  CUtensorMap tmaps[13];
   // FILTER_VARS xy pass (non-periodic FP64 grids, nx even): the state
   // buffers in 44x44x1 boxes
   bool ftma = false;
@@ -258,7 +259,7 @@ struct Handle {
   // device bookkeeping
   int *d_err = nullptr;
   long long *d_iter = nullptr, *d_fail = nullptr;
-  double *d_partials = nullptr, *d_diag = nullptr;
+  double *d_partials = nullptr, *d_diag = nullptr, *d_kseg = nullptr;
   unsigned int *d_counter = nullptr;
   int max_stage_blocks = 0;
   // FP64 MHD stages as one persistent launch (step.cu:mhd64_plan): the

@@ -28,6 +28,10 @@ __device__ __forceinline__ R dcoef(int r, int m);
 
 // geometry of the MHD stage tile (precision independent)
 namespace mg {
+// The KE norm is summed over segments of KSEG layers of a tile, so that it
+// does not depend on the z chunks (multiples of KSEG; another extent splits
+// the segments it cuts in two parts).
+constexpr int KSEG = 4;
 constexpr int TX = 32, TY = 8, NC = TX * TY, NT = 2 * NC;
 constexpr int HX = TX + 10, HY = TY + 10, HS = HX * HY;
 constexpr int NH = 10, NO = 24;
@@ -75,9 +79,9 @@ struct MhdBuf {
 // of one field's 32 x 8 own points [0..2], of all fields' [3..5] and of seven
 // fields' halo planes [6..8]; the packed background (nx, ny, nz, 18) in boxes
 // of 13 arrays' own points [9], of one's [10] and of the three B0 halo
-// planes [11]
+// planes [11] and of the three B0 own points [12]
 struct TmaSet {
-  CUtensorMap m[12];
+  CUtensorMap m[13];
 };
 
 template <class R>
@@ -331,6 +335,72 @@ __device__ void diag_reduce_t(const SimT<R> &S, double ke, double mr, double mp,
   }
 }
 
+// The same for the MHD stages of one handle: the KE norm from the segment
+// sums (S.kseg, two parts of `tiles` values per segment), the minima per item.
+template <class R>
+__device__ void diag_reduce_mhd(const SimT<R> &S, double mr, double mp, long long bid,
+                                long long nb, int tiles, int zchunk) {
+  __shared__ double r[3][32];
+  __shared__ int am_last;
+  const int nt = blockDim.x * blockDim.y * blockDim.z;
+  const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5, nw = (nt + 31) >> 5;
+  auto reduce = [&](double &ke) {  // the result in warp 0, lane 0
+    for (int o = 16; o > 0; o >>= 1) {
+      ke += __shfl_down_sync(0xffffffffu, ke, o);
+      mr = fmin(mr, __shfl_down_sync(0xffffffffu, mr, o));
+      mp = fmin(mp, __shfl_down_sync(0xffffffffu, mp, o));
+    }
+    __syncthreads();
+    if (lane == 0) { r[0][warp] = ke; r[1][warp] = mr; r[2][warp] = mp; }
+    __syncthreads();
+    if (tid == 0) {
+      ke = 0.0; mr = 1e300; mp = 1e300;
+      for (int w = 0; w < nw; ++w) {
+        ke += r[0][w]; mr = fmin(mr, r[1][w]); mp = fmin(mp, r[2][w]);
+      }
+    }
+  };
+  double ke = 0.0;
+  reduce(ke);
+  if (tid == 0) {
+    S.partials[2 * bid] = mr;
+    S.partials[2 * bid + 1] = mp;
+    __threadfence();
+    am_last = atomicAdd(S.counter, 1u) == (unsigned)(nb - 1);
+  }
+  __syncthreads();
+  if (!am_last) return;
+  __threadfence();
+  mr = 1e300; mp = 1e300;
+  for (long long b = tid; b < nb; b += nt) {
+    mr = fmin(mr, __ldcg(S.partials + 2 * b));
+    mp = fmin(mp, __ldcg(S.partials + 2 * b + 1));
+  }
+  const long long n = (long long)tiles * ((S.nz + mg::KSEG - 1) / mg::KSEG);
+  for (long long q = tid; q < n; q += nt) {
+    const long long seg = q / tiles, at = 2 * seg * tiles + (q - seg * tiles);
+    const int l0 = (int)seg * mg::KSEG, l1 = min(l0 + mg::KSEG, S.nz) - 1;
+    double v = __ldcg(S.kseg + at);
+    if (l0 / zchunk != l1 / zchunk) v += __ldcg(S.kseg + at + tiles);
+    ke += v;
+  }
+  reduce(ke);
+  if (tid == 0) {
+    const long long it = *S.iter;
+    const double nrm = sqrt(ke / ((double)S.nx * (double)S.ny * (double)S.nz));
+    const double kev = nrm * S.dimc2rho;
+    S.diag[0] = kev;
+    S.diag[1] = mr;
+    S.diag[2] = mp;
+    S.diag[3] = (double)it;
+    const bool fail = !(kev <= 1000.0) || !(mr > 0.0) || !(mp > 0.0);
+    if (fail && *S.fail_iter < 0) *S.fail_iter = it;
+    *S.iter = it + 1;
+    *S.counter = 0u;
+  }
+}
+
 // Tiles away from every edge, CPML slab and periodic wrap: their x/y
 // derivatives are the centred stencil with no branch.
 template <class R>
@@ -379,7 +449,8 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
                                          const R *__restrict__ tin,
                                          R *__restrict__ so, R beta, R bnext,
                                          int x0, int y0, int k0, int k1, int mt, int ma,
-                                         double &ke, double &mr, double &mp, uint32_t tw = 0) {
+                                         double &ke, double &mr, double &mp, uint32_t tw = 0,
+                                         double *kseg = nullptr, int kstride = 0) {
   static_assert(!TW || sizeof(R) == 8, "TMEM windows of FP64 values");
   using namespace mg;
   static_assert(TMA || !TH, "halo boxes come with the own-point boxes");
@@ -643,6 +714,13 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   // the head of layer kk + 5 is loaded a layer before layer kk needs it (into
   // q), and brought into L2 two layers before that
   auto prefetch = [&](int kk) {
+    if (TMA) {  // one box of the own points of all fields, one of B0
+      if (kk < nz && tx == 0) {
+        if (tid == 6 * 32) tma4d_l2(&T->m[3 + mt], x0, y0, kk, 0);
+        if (tid == 7 * 32) tma4d_l2(&T->m[12], x0, y0, kk, PK_BOX);
+      }
+      return;
+    }
     if (!act || kk >= nz) return;
     const int id = kk * NXY + col;
     if (role == 0) {
@@ -1010,6 +1088,19 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       if (act && role == 1) {
         const double m = ((double)O(b, O_BG + B_RHO0) + an_rho) * VSQ(b) / 2.0;
         ke += m * m;
+      }
+      if (kseg && role == 1 && ((k & (KSEG - 1)) == KSEG - 1 || k == k1 - 1)) {
+        __shared__ double kw[TY];
+        for (int o = 16; o > 0; o >>= 1) ke += __shfl_down_sync(0xffffffffu, ke, o);
+        if (tx == 0) kw[ty] = ke;
+        asm volatile("bar.sync 9, 256;" ::: "memory");  // role 1
+        if (cid == 0) {
+          double t = 0.0;
+          for (int w = 0; w < TY; ++w) t += kw[w];
+          const int seg = k / KSEG, part = seg * KSEG < k0 ? 1 : 0;
+          kseg[(long long)(2 * seg + part) * kstride] = t;
+        }
+        ke = 0.0;
       }
     }
   }

@@ -13,9 +13,11 @@
 // HBM traffic is that of the reference's scheme (14 V words per point and
 // step) and the values are bitwise those of forming a + beta*F on load.
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 
 #include "filter_body.cuh"
 #include "mhd_body.cuh"
@@ -99,24 +101,64 @@ static int quiet_zchunk(const Handle *h) {
   return best;
 }
 
+// Layers per z chunk of the MHD kernels: the extent whose items, taken by
+// one block per SM in the kernels' order (edge/CPML tiles first), finish
+// first, where an item costs its layers and two more (window loads, start)
+// and a layer of an edge tile one and a half of an interior one's time
+// (measured: 9,600 against 6,100 cycles in FP64, 6,100 against 4,150 in
+// FP32).  Against at most 40 layers in about seven blocks per SM: FP64
+// 40x40x48 0.505 -> 0.184 ms per iteration (4 layers), 149x151x203 4.98 ->
+// 4.78 (68), FP32 149x149x211 3.07 -> 2.95 (36), 128x160x180 1.77 -> 1.74
+// (32).
+static int mhd_zchunk(const Handle *h) {
+  constexpr int SMS = 148, ROUNDS = 24;
+  const sparc_params &P = h->P;
+  const bool hp = h->use_hpml;
+  const int np[4] = {hp ? P.npml_xb : 0, hp ? P.npml_xt : 0, hp ? P.npml_yb : 0,
+                     hp ? P.npml_yt : 0};
+  int ix0, ix1, iy0, iy1;
+  mhd_interior_rect(h->nx, h->ny, np, ix0, ix1, iy0, iy1);
+  const int tiles = ((h->nx + mg::TX - 1) / mg::TX) * ((h->ny + mg::TY - 1) / mg::TY);
+  const int nint = ix1 > ix0 && iy1 > iy0 ? (ix1 - ix0) * (iy1 - iy0) : 0, ngen = tiles - nint;
+  // without tensor copies an interior FP64 layer costs as much as an edge one
+  const double ratio = !h->fp32 && (h->nx & 1) ? 1.15 : 1.5;
+  int best = std::min(h->nz, 40), last = 0;
+  double least = 1e300;
+  for (int n = 1; n <= h->nz / mg::KSEG; ++n) {
+    const int zc = ((h->nz + n - 1) / n + mg::KSEG - 1) / mg::KSEG * mg::KSEG;
+    const int nch = (h->nz + zc - 1) / zc;
+    if (zc == last || zc > 160) continue;
+    last = zc;
+    if ((long long)tiles * nch > SMS * ROUNDS && n > 1) break;
+    std::vector<double> free_at(SMS, 0.0);  // a heap, the earliest in front
+    double end = 0.0;
+    for (int part = 0; part < 2; ++part)
+      for (int c = 0; c < nch; ++c) {
+        const double cost = (std::min(zc, h->nz - c * zc) + 2) * (part == 0 ? ratio : 1.0);
+        for (int t = 0; t < (part == 0 ? ngen : nint); ++t) {
+          std::pop_heap(free_at.begin(), free_at.end(), std::greater<double>());
+          free_at.back() += cost;
+          end = std::max(end, free_at.back());
+          std::push_heap(free_at.begin(), free_at.end(), std::greater<double>());
+        }
+      }
+    // extents come longest first; a shorter one has to gain 1 %
+    if (end < 0.99 * least) {
+      least = end;
+      best = zc;
+    }
+  }
+  return best;
+}
+
 int stage_geometry(Handle *h) {
   const long long tiles = (long long)((h->nx + 31) / 32) * ((h->ny + 7) / 8);
   int zc;
-  if (h->magnetic) {
-    // about seven CTAs per SM on 148 SMs (one MHD CTA is resident per SM:
-    // shorter tails; each chunk pays 10 window warm-up layers), at most 40
-    // layers (swept 30..60 on the 256x256x300 flux tube in both precisions:
-    // 40 best, 60 1.5-2 % slower, 30 1-3 % slower)
-    const long long chunks = std::max<long long>(1, (148LL * 7 + tiles - 1) / tiles);
-    zc = (int)std::max<long long>(16, (h->nz + chunks - 1) / chunks);
-    zc = std::min(zc, 40);
-  } else {
-    zc = quiet_zchunk(h);
-  }
+  zc = h->magnetic ? mhd_zchunk(h) : quiet_zchunk(h);
   zc = std::min(zc, h->nz);
   if (const char *kv = std::getenv("SPARC_ZCHUNK")) {  // A/B timing only
     const int v = std::atoi(kv);
-    if (v >= 1) zc = std::min(v, h->nz);
+    if (v >= 4) zc = std::min(v, h->nz);
   }
   h->zchunk = zc;
   h->max_stage_blocks = (int)(tiles * ((h->nz + zc - 1) / zc));
@@ -251,7 +293,8 @@ bool encode_stage_maps(Handle *h, int hxl) {
   }
   return ok && one(&h->tmaps[9], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 13) &&
          one(&h->tmaps[10], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 1) &&
-         one(&h->tmaps[11], h->bg_pack, PK_COUNT, hxl, mg::HY, 3);
+         one(&h->tmaps[11], h->bg_pack, PK_COUNT, hxl, mg::HY, 3) &&
+         one(&h->tmaps[12], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 3);
 }
 
 // ------------------------- MP_MHD_3D, shared-body stage kernel
@@ -310,14 +353,18 @@ __global__ void __launch_bounds__(mg::NT, 1)
     // the body's first barrier orders every thread's read of s_w before
     // thread 0 takes the next item
     double ke = 0.0, mr = 1e300, mp = 1e300;
+    const int tiles = ngen + nint;
+    double *kseg = S.kseg + (y0 / mg::TY) * ((S.nx + mg::TX - 1) / mg::TX) + x0 / mg::TX;
     if (in)
-      ok = mhd_body<double, MODE, TMA, true, TMA, true>(S, &T, smem, a, tin, so, beta, bnext, x0, y0,
-                                                   k0, k1, mt, ma, ke, mr, mp, tw);
+      ok = mhd_body<double, MODE, TMA, true, TMA, true>(S, &T, smem, a, tin, so, beta, bnext, x0,
+                                                        y0, k0, k1, mt, ma, ke, mr, mp, tw, kseg,
+                                                        tiles);
     else
       ok = mhd_body<double, MODE, TMA, false, TH, true>(S, &T, smem, a, tin, so, beta, bnext, x0,
-                                                    y0, k0, k1, mt, ma, ke, mr, mp, tw);
+                                                        y0, k0, k1, mt, ma, ke, mr, mp, tw, kseg,
+                                                        tiles);
     if (!ok) break;
-    if (MODE == F_LAST) diag_reduce_t(S, ke, mr, mp, w, total);
+    if (MODE == F_LAST) diag_reduce_mhd(S, mr, mp, w, total, tiles, zchunk);
   }
   __syncwarp();
   tm_wait_st();
@@ -690,6 +737,7 @@ SimDev make_simdev(Handle *h) {
   S.iter = h->d_iter;
   S.err = h->d_err;
   S.partials = h->d_partials;
+  S.kseg = h->d_kseg;
   S.counter = h->d_counter;
   S.diag = h->d_diag;
   S.fail_iter = h->d_fail;

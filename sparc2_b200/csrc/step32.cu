@@ -129,11 +129,12 @@ __global__ void __launch_bounds__(t32::NT, 1)
   double ke = 0.0, mr = 1e300, mp = 1e300;
   const int k0 = blockIdx.z * zchunk;
   if (!mhd_body<float, MODE, TMA, INT, TH>(S, &T, smem, a, tin, so, beta, bnext, x0, y0, k0,
-                                       min(S.nz, k0 + zchunk), mt, ma, ke, mr, mp))
+                                       min(S.nz, k0 + zchunk), mt, ma, ke, mr, mp, 0,
+                                       S.kseg + tx_ + (long long)gx * ty_, gx * gy))
     return;
   if (MODE == F_LAST)
-    diag_reduce_t(S, ke, mr, mp, tx_ + (long long)gx * (ty_ + (long long)gy * blockIdx.z),
-                  (long long)gx * gy * gridDim.z);
+    diag_reduce_mhd(S, mr, mp, tx_ + (long long)gx * (ty_ + (long long)gy * blockIdx.z),
+                    (long long)gx * gy * gridDim.z, gx * gy, zchunk);
 }
 
 // ---------------------------------------------- FILTER_VARS, precision form
@@ -353,6 +354,7 @@ Sim32 make_sim32(Handle *h) {
   S.iter = h->d_iter;
   S.err = h->d_err;
   S.partials = h->d_partials;
+  S.kseg = h->d_kseg;
   S.counter = h->d_counter;
   S.diag = h->d_diag;
   S.fail_iter = h->d_fail;

@@ -42,6 +42,12 @@ __device__ __forceinline__ void tma4d_t(void *dst, const CUtensorMap *map, int x
       "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(sm_addr_t(bar))
       : "memory");
 }
+// brings the 4-D tile into L2 (no shared memory, no completion)
+__device__ __forceinline__ void tma4d_l2(const CUtensorMap *map, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(map),
+               "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
 // bounded wait: gives up after kMbarWaitLimit polls and raises the error flag
 __device__ __forceinline__ bool mbar_wait_t(unsigned long long *bar, unsigned parity, int *err) {
   for (long long n = 0; n < kMbarWaitLimit; ++n) {
