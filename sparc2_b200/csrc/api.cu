@@ -144,8 +144,8 @@ static int alloc_face(Handle *h, int f, int n0, int n1, int n2, int np) {
 static int zero_state(Handle *h) {
   if (h->fp32) {
     for (int b = 0; b < 3; ++b)
-      CK(h, cudaMemsetAsync(h->fbuf[b], 0, (size_t)h->V * h->N * 4, h->stream));
-    CK(h, cudaMemsetAsync(h->f_carry, 0, (size_t)h->V * h->N * 4, h->stream));
+      CK(h, cudaMemsetAsync(h->fbuf[b], 0, (size_t)h->V * h->NP * 4, h->stream));
+    CK(h, cudaMemsetAsync(h->f_carry, 0, (size_t)h->V * h->NP * 4, h->stream));
     for (auto &F : h->f_faces)
       if (F.on) {
         CK(h, cudaMemsetAsync(F.vars, 0, F.cnt * F.P * 4, h->stream));
@@ -154,7 +154,7 @@ static int zero_state(Handle *h) {
     return SPARC_OK;
   }
   for (int b = 0; b < 3; ++b)
-    CK(h, cudaMemsetAsync(h->buf[b], 0, (size_t)h->V * h->N * 8, h->stream));
+    CK(h, cudaMemsetAsync(h->buf[b], 0, (size_t)h->V * h->NP * 8, h->stream));
   for (auto &F : h->faces)
     if (F.on) {
       CK(h, cudaMemsetAsync(F.vars, 0, F.cnt * F.P * 8, h->stream));
@@ -245,7 +245,7 @@ static int enqueue_filter32(Handle *h, int fk, cudaStream_t s, int *nk) {
     rotate(h);
     ++*nk;
   }
-  if (fk && cudaMemsetAsync(h->f_carry, 0, (size_t)h->V * h->N * 4, s) != cudaSuccess)
+  if (fk && cudaMemsetAsync(h->f_carry, 0, (size_t)h->V * h->NP * 4, s) != cudaSuccess)
     r = SPARC_ERR_CUDA;
   return r ? SPARC_ERR_CUDA : SPARC_OK;
 }
@@ -395,6 +395,13 @@ int sparc_create(const sparc_params *p, int device, sparc_handle **out) {
     h->xaxis[i] = h->periodic ? (double)i / (double)h->nx : (double)i / (double)(h->nx - 1);
   for (int j = 0; j < h->ny; ++j)
     h->yaxis[j] = h->periodic ? (double)j / (double)h->ny : (double)j / (double)(h->ny - 1);
+  h->px = h->nx;
+  if (h->magnetic) {
+    const int q = h->fp32 ? 4 : 2, px = (h->nx + q - 1) / q * q;
+    // (the stage kernels index the eight fields with 32 bits)
+    if ((long long)px * h->ny * h->nz * 8 < (1LL << 31)) h->px = px;
+  }
+  h->NP = (long long)h->px * h->ny * h->nz;
   h->stretchx = h->periodic ? RSUN / p->xlength * h->nx : RSUN / p->xlength * (h->nx - 1);
   h->stretchy = h->periodic ? RSUN / p->ylength * h->ny : RSUN / p->ylength * (h->ny - 1);
   block_partition(h->nx, p->block_x, h->bxs, h->bxl);
@@ -456,15 +463,15 @@ int sparc_create(const sparc_params *p, int device, sparc_handle **out) {
   for (int b = 0; !r && b < 3; ++b) {
     if (h->fp32) {
       // (the free buffers hold half of the FP64 state each in state I/O)
-      h->fbuf[b] = (float *)dev_alloc(h, ((size_t)h->V * h->N + 1) / 2 * 8);
+      h->fbuf[b] = (float *)dev_alloc(h, ((size_t)h->V * h->NP + 1) / 2 * 8);
       if (!h->fbuf[b]) r = SPARC_ERR_NOMEM;
     } else {
-      h->buf[b] = (double *)dev_alloc(h, (size_t)h->V * h->N * 8);
+      h->buf[b] = (double *)dev_alloc(h, (size_t)h->V * h->NP * 8);
       if (!h->buf[b]) r = SPARC_ERR_NOMEM;
     }
   }
   if (!r && h->fp32) {
-    h->f_carry = (float *)dev_alloc(h, (size_t)h->V * h->N * 4);
+    h->f_carry = (float *)dev_alloc(h, (size_t)h->V * h->NP * 4);
     if (!h->f_carry) r = SPARC_ERR_NOMEM;
   }
   if (!r && h->use_pml) {
@@ -758,7 +765,7 @@ int sparc_set_state(sparc_handle *h, const double *a, const double *psi) {
     return SPARC_OK;
   }
   int r;
-  if (a && (r = state_to_device(h, h->buf[h->ra], a, (size_t)h->V * h->N))) return r;
+  if (a && (r = set_state64(h, a))) return r;
   if (psi)
     for (auto &F : h->faces)
       if (F.on) {
@@ -792,7 +799,7 @@ int sparc_get_state(sparc_handle *h, double *a, double *psi) {
     return get_state32(h, a, psi);
   }
   int r;
-  if (a && (r = state_to_host(h, a, h->buf[h->ra], (size_t)h->V * h->N))) return r;
+  if (a && (r = get_state64(h, a))) return r;
   if (psi)
     for (auto &F : h->faces)
       if (F.on) {
@@ -1092,7 +1099,11 @@ int sparc_get_coeff(sparc_handle *h, const char *name, double *out,
   }
   if (!dsrc) return fail(h, SPARC_ERR_INVALID, "coefficient not used in this mode");
   *count = n;
-  if (out) CK(h, cudaMemcpy(out, dsrc, n * 8, cudaMemcpyDeviceToHost));
+  const double *pk = (const double *)h->bg_pack;
+  const int pitch = pk && dsrc >= pk && dsrc < pk + PK_COUNT * h->NP ? h->px : h->nx;
+  if (out)
+    CK(h, cudaMemcpy2D(out, (size_t)h->nx * 8, dsrc, (size_t)pitch * 8, (size_t)h->nx * 8,
+                       (size_t)h->ny * h->nz, cudaMemcpyDeviceToHost));
   return SPARC_OK;
 }
 

@@ -136,7 +136,7 @@ int rebuild(Batch *b) {
     Handle *h = b->members[q];
     if (!h) continue;
     Slot32 &L = b->slots[q];
-    const long long tot = (long long)h->V * h->N;
+    const long long tot = (long long)h->V * h->NP;
     L.f_first = (int)fitems.size();
     for (long long t = 0; t < tot; t += b->fchunk)
       fitems.push_back(make_int4(q, (int)t, (int)std::min<long long>(b->fchunk, tot - t), 0));

@@ -63,17 +63,18 @@ int damping_setup(Handle *h) {
   }
   h->d_damp = (double *)dev_alloc(h, rates.size() * 8);
   h->d_spec = (double2 *)dev_alloc(h, (size_t)nh * ny * nz * sizeof(double2));
-  h->d_term = (double *)dev_alloc(h, (size_t)3 * h->N * 8);
+  h->d_term = (double *)dev_alloc(h, (size_t)3 * h->NP * 8);
   if (!h->d_damp || !h->d_spec || !h->d_term) return SPARC_ERR_NOMEM;
   if (cudaMemcpyAsync(h->d_damp, rates.data(), rates.size() * 8, cudaMemcpyHostToDevice,
                       h->stream) != cudaSuccess ||
       cudaStreamSynchronize(h->stream) != cudaSuccess)
     return SPARC_ERR_CUDA;
-  int n[2] = {ny, nx}, real_e[2] = {ny, nx}, half_e[2] = {ny, nh};
-  if (!fft_ok(h, cufftPlanMany(&h->fft_fwd, 2, n, real_e, 1, nx * ny, half_e, 1, nh * ny,
+  // (real rows are px values apart, as in the state)
+  int n[2] = {ny, nx}, real_e[2] = {ny, h->px}, half_e[2] = {ny, nh};
+  if (!fft_ok(h, cufftPlanMany(&h->fft_fwd, 2, n, real_e, 1, h->px * ny, half_e, 1, nh * ny,
                                CUFFT_D2Z, nz),
               "cufftPlanMany (forward)") ||
-      !fft_ok(h, cufftPlanMany(&h->fft_inv, 2, n, half_e, 1, nh * ny, real_e, 1, nx * ny,
+      !fft_ok(h, cufftPlanMany(&h->fft_inv, 2, n, half_e, 1, nh * ny, real_e, 1, h->px * ny,
                                CUFFT_Z2D, nz),
               "cufftPlanMany (inverse)"))
     return SPARC_ERR_CUDA;
@@ -91,14 +92,14 @@ int damping_enqueue(Handle *h, const double *tin, cudaStream_t s) {
     return SPARC_ERR_CUDA;
   for (int l = 0; l < 3; ++l) {
     // the forward transform does not write its input (out of place)
-    double *in = const_cast<double *>(tin) + (size_t)(l + 1) * h->N;
+    double *in = const_cast<double *>(tin) + (size_t)(l + 1) * h->NP;
     if (!fft_ok(h, cufftExecD2Z(h->fft_fwd, in, (cufftDoubleComplex *)h->d_spec),
                 "cufftExecD2Z"))
       return SPARC_ERR_CUDA;
     k_damp_mul<<<blocks, 256, 0, s>>>(h->d_spec, h->d_damp, nh, total);
     ++h->launches;
     if (!fft_ok(h, cufftExecZ2D(h->fft_inv, (cufftDoubleComplex *)h->d_spec,
-                                h->d_term + (size_t)l * h->N),
+                                h->d_term + (size_t)l * h->NP),
                 "cufftExecZ2D"))
       return SPARC_ERR_CUDA;
   }

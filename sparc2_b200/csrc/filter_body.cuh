@@ -51,7 +51,8 @@ constexpr size_t filt_z_smem();
 template <class R>
 struct FiltArgs {
   int nx, ny, nz, V;
-  long long N;
+  int px;             // row pitch
+  long long N;        // px * ny * nz
   int periodic;
   R s;                // a - s*filt (7-point filter)
   const R *in;
@@ -143,10 +144,10 @@ __device__ __forceinline__ void filt_xy_tile(const FiltArgs<R> &F, int l, int k,
   __shared__ R raw[RY][RX];  // rows y0-6 .., columns x0-6 ..
   __shared__ R fy[TR][RX];   // after the y pass, rows y0 .., columns x0-6 ..
   const int tid = threadIdx.y * TX + threadIdx.x;
-  const int nx = F.nx, ny = F.ny;
+  const int nx = F.nx, ny = F.ny, px = F.px;
   const bool per = F.periodic;
   const R fs = F.s;
-  const long long base = (long long)l * F.N + (long long)k * nx * ny;
+  const long long base = (long long)l * F.N + (long long)k * px * ny;
   const R *in = F.in + base;
   const R *cin = CARRY ? F.carry + base : nullptr;
   // the (32+12) x (32+12) neighbourhood, one flat index over it
@@ -162,7 +163,7 @@ __device__ __forceinline__ void filt_xy_tile(const FiltArgs<R> &F, int l, int k,
     }
     R v = R(0);
     if (ok) {
-      const int id = gy * nx + gx;
+      const int id = gy * px + gx;
       v = in[id];
       if (CARRY) v = v - cin[id];
     }
@@ -213,7 +214,7 @@ __device__ __forceinline__ void filt_xy_tile(const FiltArgs<R> &F, int l, int k,
     const R *c = &fy[r][tx + 6];
     const R pq = *c;
     const R filt = (!per && (gxo < G || gxo >= nx - G)) ? (M2 ? R(0) : pq) : ftaps<R, G>(c, 1);
-    out[gyo * nx + gxo] = M2 ? pq - fs * filt : filt;
+    out[gyo * px + gxo] = M2 ? pq - fs * filt : filt;
   }
 }
 
@@ -254,10 +255,10 @@ __device__ __forceinline__ void filt_xy_layers(const FiltArgs<R> &F, int l, int 
   __shared__ R fy[TR][RX];       // after the y pass, rows y0 .., columns x0-6 ..
   __shared__ unsigned long long fbar[2];
   const int tid = threadIdx.y * TX + threadIdx.x;
-  const int nx = F.nx, ny = F.ny;
+  const int nx = F.nx, ny = F.ny, px = F.px;
   const bool per = F.periodic;
   const R fs = F.s;
-  const long long NXY = (long long)nx * ny;
+  const long long NXY = (long long)px * ny;
   const R *inl = F.in + (long long)l * F.N;
   R *outl = F.out + (long long)l * F.N;
   if constexpr (TMA) {
@@ -290,7 +291,7 @@ __device__ __forceinline__ void filt_xy_layers(const FiltArgs<R> &F, int l, int 
         } else {
           ok = gy >= 0 && gy < ny && gx >= 0 && gx < nx;
         }
-        filt_cp(&raw2[b][ry][rx], ok ? in + gy * nx + gx : in, ok);
+        filt_cp(&raw2[b][ry][rx], ok ? in + gy * px + gx : in, ok);
       }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
@@ -357,7 +358,7 @@ __device__ __forceinline__ void filt_xy_layers(const FiltArgs<R> &F, int l, int 
       const R pq = *c;
       const R filt =
           (!per && (gxo < G || gxo >= nx - G)) ? (M2 ? R(0) : pq) : ftaps<R, G>(c, 1);
-      out[gyo * nx + gxo] = M2 ? pq - fs * filt : filt;
+      out[gyo * px + gxo] = M2 ? pq - fs * filt : filt;
     }
   }
 }
@@ -382,11 +383,11 @@ __device__ __forceinline__ void filt_z_slab(const FiltArgs<R> &F, int l, int x0,
   static_assert(!TMA || (!CARRY && !SC), "the tensor copy moves stored values only");
   const int tx = threadIdx.x, ty = threadIdx.y, tz = threadIdx.z;
   const int nx = F.nx, ny = F.ny, nz = F.nz;
-  const long long NXY = (long long)nx * ny;
+  const long long NXY = (long long)F.px * ny;
   const int gx = x0 + tx, gy = y0 + ty;
   const bool colok = gx < nx && gy < ny;
   // this thread's column; each thread loads layers q = tz, tz + 2, ...
-  const R *icol = F.in + (long long)l * F.N + (colok ? (long long)gy * nx + gx : 0);
+  const R *icol = F.in + (long long)l * F.N + (colok ? (long long)gy * F.px + gx : 0);
   if constexpr (TMA) {
     // the mbarrier follows the slab in the dynamic buffer (a static one
     // would cost a kilobyte of the CTA's shared allocation)

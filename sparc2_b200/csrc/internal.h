@@ -59,7 +59,8 @@ using ForcingDev = ForcingT<double>;
 template <class R>
 struct SimT {
   int nx, ny, nz;
-  long long N;
+  int px;                      // row pitch of the state and 3-D background arrays
+  long long N;                 // values of such an array: px * ny * nz
   int periodic, magnetic, bg1d;
   int sponge_slabs;            // the sponge vanishes outside the CPML slabs
   int V;
@@ -176,6 +177,12 @@ struct Handle {
   int device = 0;
   int nx = 0, ny = 0, nz = 0, V = 0, Pp = 0;
   long long N = 0;
+  // Rows of the state and of the packed background are px values apart: the
+  // next multiple of 16 bytes for MHD (every nx then has tensor copies, whose
+  // rows must start there), nx for the quiet equations.  NP = px * ny * nz.
+  // Columns past nx are never read.
+  int px = 0;
+  long long NP = 0;
   bool magnetic = false, quiet = false, periodic = false;
   bool use_pml = false, use_hpml = false;
   int gxy = 5, gz = 5, xyfreq = 1, zfreq = 1;
@@ -332,6 +339,8 @@ int launch_filter_event(Handle *h, bool xy, const double *in, double *out, cudaS
 int stage_geometry(Handle *h);
 int encode_tensor_maps(Handle *h);
 bool encode_stage_maps(Handle *h, int hxl);
+int repitch(const double *src, int sp, double *dst, int dp, int nx, long long rows,
+            cudaStream_t s);
 
 // step32.cu (precision form)
 int step32_constants();
@@ -361,6 +370,8 @@ void state_io_open();
 void state_io_close();
 int state_to_host(Handle *h, double *host, const void *dev, size_t count);
 int state_to_device(Handle *h, void *dev, const double *host, size_t count);
+int set_state64(Handle *h, const double *a);
+int get_state64(Handle *h, double *a);
 int set_state32(Handle *h, const double *a, const double *psi);
 int get_state32(Handle *h, double *a, double *psi);
 

@@ -123,12 +123,13 @@ __device__ __forceinline__ int origin_t(int t0, int T, int n, bool per) {
   return o;
 }
 
-// the same where the halo rows are TMA boxes: the box starts XOFF columns
-// earlier, at a multiple of 16 bytes (n is even in FP64, a multiple of 4 in
-// FP32, so n - 12 and n - 16 are)
+// the same where the halo rows are TMA boxes, which start XOFF columns earlier
+// at a multiple of 16 bytes: the last tile's origin is the largest such one
+// that has f(n-11..n-1) in the tile
 template <class R>
 __host__ __device__ __forceinline__ int origin_th(int t0, int T, int n) {
-  const int o = t0 - 5, e = sizeof(R) == 8 ? n - 11 : n - 13;
+  constexpr int A = 16 / (int)sizeof(R), XOFF = sizeof(R) == 8 ? 1 : 3;
+  const int o = t0 - 5, e = (n - 11 - XOFF) / A * A + XOFF;
   return t0 + T >= n && e < o ? e : o;
 }
 
@@ -461,11 +462,11 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   const int tx = threadIdx.x, ty = threadIdx.y, role = threadIdx.z;
   const int tid = (role * TY + ty) * TX + tx, cid = ty * TX + tx;
   const int nx = S.nx, ny = S.ny, nz = S.nz;
-  const int N = (int)S.N, NXY = nx * ny;
+  const int px = S.px, N = (int)S.N, NXY = px * ny;
   const int i = x0 + tx, j = y0 + ty;
   const bool act = INT || (i < nx && j < ny);
   const bool per = S.periodic;
-  const int col = j * nx + i;
+  const int col = j * px + i;
   const int xo = INT ? x0 - 5 : (TH ? origin_th<R>(x0, TX, nx) : origin_t(x0, TX, nx, per));
   const int yo = INT ? y0 - 5 : origin_t(y0, TY, ny, per);
   const int ry = y0 - yo + ty, rx = x0 - xo + tx;
@@ -569,7 +570,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       }
       if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) return;
       hs = ly * HXL + lx;
-      ho = gy * nx + gx;
+      ho = gy * px + gx;
     };
     auto yrow = [&](int h, int &hs, int &ho) { pos(rx, h < cy0 ? h : h + TY, hs, ho); };
     if (role == 0) {
@@ -580,7 +581,10 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
         yrow(8 + ty, hs1, ho1);
       } else if (cid < 64 + 10 * TY) {
         const int q = cid - 64, r = q / 10, c = q - r * 10;
-        pos(c < cx0 ? c : c + TX, cy0 + r, hs1, ho1);
+        // (a last tile whose origin moved down by more than five columns has
+        // the ten before it)
+        const int cl = min(cx0, 10);
+        pos(c < cl ? c + cx0 - cl : c + TX, cy0 + r, hs1, ho1);
       }
     }
   }
@@ -773,6 +777,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   const bool xbot = i < S.xb.np, ybot = j < S.yb.np;
   const bool xpml = !INT && S.xb.on && act && (xbot || i >= nx - S.xt.np);
   const bool ypml = !INT && S.yb.on && act && (ybot || j >= ny - S.yt.np);
+  auto face_z = [&](int kl) -> long long { return ((long long)kl * ny + j) * nx + i; };
   auto face_x = [&](int k) -> long long {
     const int np = xbot ? S.xb.np : S.xt.np;
     return (xbot ? i : i - (nx - np)) + (long long)np * (j + (long long)ny * k);
@@ -824,7 +829,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       if (zpml && act) {
         const bool bot = k < S.zb.np;
         const int kl = bot ? k : k - (nz - S.zt.np);
-        pf_face(bot ? S.zb : S.zt, (long long)kl * NXY + col, kl, role ? 4 : 1, role ? 5 : 2,
+        pf_face(bot ? S.zb : S.zt, face_z(kl), kl, role ? 4 : 1, role ? 5 : 2,
                 role ? 0 : 3);
       }
       if (xpml) pf_face(xbot ? S.xb : S.xt, face_x(k), 0, role ? 0 : 1, role ? 4 : 3,
@@ -937,9 +942,9 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       const bool bot = k < S.zb.np;
       const FaceT<R> &F = bot ? S.zb : S.zt;
       const int kl = bot ? k : k - (nz - S.zt.np);
-      cpml3_t<R, MODE>(F, (long long)kl * NXY + col, kl, s0, s1, s2, beta, dt, da, db, dc);
+      cpml3_t<R, MODE>(F, face_z(kl), kl, s0, s1, s2, beta, dt, da, db, dc);
     };
-    auto px = [&](int s0, int s1, int s2, R &da, R &db, R &dc) {
+    auto pmlx = [&](int s0, int s1, int s2, R &da, R &db, R &dc) {
       cpml3_t<R, MODE>(xbot ? S.xb : S.xt, face_x(k), 0, s0, s1, s2, beta, dt, da, db, dc);
     };
     auto py = [&](int s0, int s1, int s2, R &da, R &db, R &dc) {
@@ -957,7 +962,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
         d1 *= ip; d4 *= ib; d8 *= ib;
         d2 = DZ(0); d6 = DZ(1); d3 = DZ(2);
         if (zpml) pz(1, 2, 3, d2, d6, d3);
-        if (xpml) px(1, 3, 2, d0, d5, d7);
+        if (xpml) pmlx(1, 3, 2, d0, d5, d7);
         if (ypml) py(1, 3, 2, d1, d4, d8);
         // curl b
         d4 = d4 - d3;
@@ -970,7 +975,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
         d1 *= iv; d4 *= iv; d5 *= iv;
         d6 = DZ(0); d7 = DZ(1); d8 = DZ(2);
         if (zpml) pz(4, 5, 0, d7, d6, d8);
-        if (xpml) px(0, 4, 5, d0, d2, d3);
+        if (xpml) pmlx(0, 4, 5, d0, d2, d3);
         if (ypml) py(0, 4, 5, d1, d4, d5);
         // curl(v x B0) and the divergence
         d4 = d4 - d7;

@@ -49,7 +49,9 @@ static unsigned char *g_noalloc_ptr[kMaxDevices] = {};
 // m = (rho0 + rho) |v|^2 / 2 at point n, from the FP64 state or from the
 // FP32 state with its carry and depth scales
 struct KeSrc {
-  long long N, NXY;
+  long long N, NXY;                      // points of the grid, of a layer
+  long long NP;                          // values of a field: rows px apart
+  int nx, px, ny;
   int nz, bg1d;
   const double *a;                       // FP64 form
   const float *fa, *carry, *isc, *frho0; // FP32 form
@@ -59,16 +61,20 @@ struct KeSrc {
 
 __device__ __forceinline__ double ke_density(const KeSrc &S, const float *fa, long long n) {
   const int k = (int)(n / S.NXY);
+  if (S.px != S.nx) {
+    const long long row = n / S.nx;
+    n = row * S.px + (n - row * S.nx);
+  }
   double r, v1, v2, v3, r0;
   if (S.a) {
     r = S.a[n];
-    v1 = S.a[S.N + n];
-    v2 = S.a[2 * S.N + n];
-    v3 = S.a[3 * S.N + n];
+    v1 = S.a[S.NP + n];
+    v2 = S.a[2 * S.NP + n];
+    v3 = S.a[3 * S.NP + n];
     r0 = S.rho0[n];
   } else {
     auto ph = [&](int l) {
-      const long long q = l * S.N + n;
+      const long long q = l * S.NP + n;
       return ((double)fa[q] - (double)S.carry[q]) * (double)S.isc[l * S.nz + k];
     };
     r = ph(0);
@@ -171,6 +177,10 @@ extern "C" int sparc_ke_norm_noalloc(sparc_handle *hh, double *ke_norm) {
   KeSrc S{};
   S.N = h->N;
   S.NXY = (long long)h->nx * h->ny;
+  S.NP = h->NP;
+  S.nx = h->nx;
+  S.px = h->px;
+  S.ny = h->ny;
   S.nz = h->nz;
   if (h->batch) {
     // the batch owns the roles: read the live one from the member's device

@@ -38,8 +38,9 @@ namespace sparc {
 // coefficients, CPML fields and profiles, forcing tables) and at the peak
 // of its set-up (plus the FP64 setup arrays released after conversion).
 void estimate_bytes32(const sparc_params &P, int64_t *resident, int64_t *peak) {
-  const long long N = (long long)P.nx * P.ny * P.nz;
   const bool mhd = P.magnetic == 2;
+  // (MHD rows are padded to 16 bytes)
+  const long long N = (long long)(mhd ? (P.nx + 3) / 4 * 4 : P.nx) * P.ny * P.nz;
   const int V = mhd ? 8 : 5, Pp = mhd ? 6 : 2;
   const bool hp = P.use_hpml != 0, pml = P.use_pml != 0 || hp;
   long long face_cnt = 0;

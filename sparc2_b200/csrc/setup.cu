@@ -359,7 +359,7 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
   // ------------------------------------------------ 3-D arrays (FP64)
   // MHD in the plain form: the arrays of the stage kernels in one allocation
   double *pack = nullptr;
-  if (h->magnetic && !h->fp32) {
+  if (h->magnetic && !h->fp32 && h->px == nx) {
     h->bg_pack = pack = up(h, nullptr, PK_COUNT * N);
     if (!pack) return SPARC_ERR_NOMEM;
   }
@@ -773,6 +773,23 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
     const double *pk = F.pk;
     each(n, s, [=] __device__(long long t) { ki[t] = 1.0 / pk[t]; });
     F.pki = ki;
+  }
+  // plain-form MHD with padded rows: the arrays set up so far, packed
+  if (h->magnetic && !h->fp32 && !pack) {
+    double **arr[PK_COUNT] = {&h->red, &h->rho0, &h->grx, &h->gry, &h->grz, &h->c2rho0,
+                              &h->gpx, &h->gpy, &h->gpz, &h->rhoinv, &h->cbx, &h->cby,
+                              &h->cbz, &h->sponge, &h->p0, &h->box, &h->boy, &h->boz};
+    pack = up(h, nullptr, PK_COUNT * h->NP);
+    if (!pack) return SPARC_ERR_NOMEM;
+    h->bg_pack = pack;
+    for (int n = 0; n < PK_COUNT; ++n)
+      if (repitch(*arr[n], nx, pack + n * h->NP, h->px, nx, (long long)ny * nz, s))
+        return SPARC_ERR_CUDA;
+    CK(cudaStreamSynchronize(s));
+    for (int n = 0; n < PK_COUNT; ++n) {
+      dev_free(h, *arr[n]);
+      *arr[n] = pack + n * h->NP;
+    }
   }
   CK(cudaStreamSynchronize(s));
   return SPARC_OK;

@@ -180,30 +180,74 @@ int state_to_device(Handle *h, void *dev, const double *host, size_t count) {
   return state_copy(h, const_cast<double *>(host), dev, count * 8, true);
 }
 
+// rows of nx values, sp apart at the source, dp apart at the destination
+__global__ void k_repitch(const double *__restrict__ src, int sp, double *__restrict__ dst, int dp,
+                          int nx, long long rows) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (long long r = (long long)blockIdx.x * nw + warp; r < rows; r += (long long)gridDim.x * nw)
+    for (int i = lane; i < nx; i += 32) dst[r * dp + i] = src[r * sp + i];
+}
+
+int repitch(const double *src, int sp, double *dst, int dp, int nx, long long rows,
+            cudaStream_t s) {
+  k_repitch<<<(unsigned)std::min<long long>((rows + 7) / 8, 148 * 16), 256, 0, s>>>(src, sp, dst,
+                                                                                  dp, nx, rows);
+  return cudaGetLastError() == cudaSuccess ? SPARC_OK : SPARC_ERR_CUDA;
+}
+
+// plain form: rows px apart on the device, packed in a free buffer on the way
+int set_state64(Handle *h, const double *a) {
+  double *st = h->buf[h->ra], *tmp = h->buf[h->rf1];
+  const size_t n = (size_t)h->V * h->N;
+  if (h->px == h->nx) return state_to_device(h, st, a, n);
+  const int r = state_to_device(h, tmp, a, n);
+  return r ? r
+           : repitch(tmp, h->nx, st, h->px, h->nx, (long long)h->V * h->ny * h->nz, h->stream);
+}
+int get_state64(Handle *h, double *a) {
+  const double *st = h->buf[h->ra];
+  double *tmp = h->buf[h->rf1];
+  if (h->px != h->nx) {
+    if (repitch(st, h->px, tmp, h->nx, h->nx, (long long)h->V * h->ny * h->nz, h->stream))
+      return SPARC_ERR_CUDA;
+    st = tmp;
+  }
+  return state_to_host(h, a, st, (size_t)h->V * h->N);
+}
+
 // ------------------------------------------------ precision form
 // Values [0, half) of the FP64 image lie in lo, the others in hi (the two
-// free state buffers).  One (field, layer) plane per block and step.
+// free state buffers).  One (field, layer) plane per block and step, a row
+// per warp; device rows are px apart.
 __global__ void k_state_out(const float *__restrict__ st, const float *__restrict__ carry,
-                            const float *__restrict__ isc, int planes, int nxy, long long half,
-                            double *__restrict__ lo, double *__restrict__ hi) {
+                            const float *__restrict__ isc, int planes, int nx, int ny, int px,
+                            long long half, double *__restrict__ lo, double *__restrict__ hi) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int p = blockIdx.x; p < planes; p += gridDim.x) {
     const double q = (double)isc[p];
-    for (int n = threadIdx.x; n < nxy; n += blockDim.x) {
-      const long long t = (long long)p * nxy + n;
-      const double v = ((double)st[t] - (double)carry[t]) * q;
-      if (t < half) lo[t] = v;
-      else hi[t - half] = v;
+    for (int j = warp; j < ny; j += nw) {
+      const long long row = (long long)p * ny + j;
+      for (int i = lane; i < nx; i += 32) {
+        const long long t = row * nx + i, d = row * px + i;
+        const double v = ((double)st[d] - (double)carry[d]) * q;
+        if (t < half) lo[t] = v;
+        else hi[t - half] = v;
+      }
     }
   }
 }
 __global__ void k_state_in(const double *__restrict__ lo, const double *__restrict__ hi,
-                           const float *__restrict__ sc, int planes, int nxy, long long half,
-                           float *__restrict__ st) {
+                           const float *__restrict__ sc, int planes, int nx, int ny, int px,
+                           long long half, float *__restrict__ st) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int p = blockIdx.x; p < planes; p += gridDim.x) {
     const double q = (double)sc[p];
-    for (int n = threadIdx.x; n < nxy; n += blockDim.x) {
-      const long long t = (long long)p * nxy + n;
-      st[t] = (float)(q * (t < half ? lo[t] : hi[t - half]));
+    for (int j = warp; j < ny; j += nw) {
+      const long long row = (long long)p * ny + j;
+      for (int i = lane; i < nx; i += 32) {
+        const long long t = row * nx + i;
+        st[row * px + i] = (float)(q * (t < half ? lo[t] : hi[t - half]));
+      }
     }
   }
 }
@@ -227,15 +271,15 @@ __global__ void k_narrow(const double *__restrict__ in, long long n, float *__re
 int set_state32(Handle *h, const double *a, const double *psi) {
   const long long VN = (long long)h->V * h->N, half = VN / 2;
   double *lo = (double *)h->fbuf[h->rf1], *hi = (double *)h->fbuf[h->rf2];
-  const int planes = h->V * h->nz, nxy = h->nx * h->ny;
+  const int planes = h->V * h->nz;
   int r;
   if (a) {
     if ((r = state_to_device(h, lo, a, half))) return r;
     if ((r = state_to_device(h, hi, a + half, VN - half))) return r;
-    k_state_in<<<std::min(planes, 148 * 16), 256, 0, h->stream>>>(lo, hi, h->f_sc, planes, nxy,
-                                                                  half, h->fbuf[h->ra]);
+    k_state_in<<<std::min(planes, 148 * 16), 256, 0, h->stream>>>(
+        lo, hi, h->f_sc, planes, h->nx, h->ny, h->px, half, h->fbuf[h->ra]);
     CKS(cudaGetLastError());
-    CKS(cudaMemsetAsync(h->f_carry, 0, (size_t)VN * 4, h->stream));
+    CKS(cudaMemsetAsync(h->f_carry, 0, (size_t)h->V * h->NP * 4, h->stream));
     CKS(cudaStreamSynchronize(h->stream));
   }
   if (psi)
@@ -255,11 +299,11 @@ int set_state32(Handle *h, const double *a, const double *psi) {
 int get_state32(Handle *h, double *a, double *psi) {
   const long long VN = (long long)h->V * h->N, half = VN / 2;
   double *lo = (double *)h->fbuf[h->rf1], *hi = (double *)h->fbuf[h->rf2];
-  const int planes = h->V * h->nz, nxy = h->nx * h->ny;
+  const int planes = h->V * h->nz;
   int r;
   if (a) {
     k_state_out<<<std::min(planes, 148 * 16), 256, 0, h->stream>>>(
-        h->fbuf[h->ra], h->f_carry, h->f_isc, planes, nxy, half, lo, hi);
+        h->fbuf[h->ra], h->f_carry, h->f_isc, planes, h->nx, h->ny, h->px, half, lo, hi);
     CKS(cudaGetLastError());
     if ((r = state_to_host(h, a, lo, half))) return r;
     if ((r = state_to_host(h, a + half, hi, VN - half))) return r;

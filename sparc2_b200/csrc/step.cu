@@ -121,7 +121,7 @@ static int mhd_zchunk(const Handle *h) {
   const int tiles = ((h->nx + mg::TX - 1) / mg::TX) * ((h->ny + mg::TY - 1) / mg::TY);
   const int nint = ix1 > ix0 && iy1 > iy0 ? (ix1 - ix0) * (iy1 - iy0) : 0, ngen = tiles - nint;
   // without tensor copies an interior FP64 layer costs as much as an edge one
-  const double ratio = !h->fp32 && (h->nx & 1) ? 1.15 : 1.5;
+  const double ratio = !h->fp32 && (h->px & 1) ? 1.15 : 1.5;
   int best = std::min(h->nz, 40), last = 0;
   double least = 1e300;
   for (int n = 1; n <= h->nz / mg::KSEG; ++n) {
@@ -198,10 +198,10 @@ int encode_tensor_maps(Handle *h) {
   h->ftma = false;
   // rows of a multiple of 16 bytes; the filter's tiles read zero outside
   // the grid, so its maps serve non-periodic grids only
-  const bool want_f = !h->periodic && !(h->nx & 1);
+  const bool want_f = !h->periodic && !(h->px & 1);
   h->ztma = false;
-  const bool want_z = !(h->nx & 1);
-  h->tma = h->magnetic && !(h->nx & 1) && h->allow_tma64 &&
+  const bool want_z = !(h->px & 1);
+  h->tma = h->magnetic && !(h->px & 1) && h->allow_tma64 &&
            encode_stage_maps(h, MhdBuf<double, true>::HXL);
   if (!want_f && !want_z) return SPARC_OK;
   void *fn = nullptr;
@@ -218,7 +218,7 @@ int encode_tensor_maps(Handle *h) {
   auto boxed = [&](CUtensorMap *m, const double *base, unsigned long long depth, int bx,
                    int by) {
     cuuint64_t dims[3] = {(cuuint64_t)h->nx, (cuuint64_t)h->ny, (cuuint64_t)depth};
-    cuuint64_t strides[2] = {(cuuint64_t)h->nx * 8, (cuuint64_t)h->nx * h->ny * 8};
+    cuuint64_t strides[2] = {(cuuint64_t)h->px * 8, (cuuint64_t)h->px * h->ny * 8};
     cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
     cuuint32_t es[3] = {1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, (void *)base, dims, strides, box, es,
@@ -242,8 +242,8 @@ int encode_tensor_maps(Handle *h) {
     for (int b = 0; b < 3 && zok; ++b) {
       cuuint64_t dims[4] = {(cuuint64_t)h->nx, (cuuint64_t)h->ny, (cuuint64_t)h->nz,
                             (cuuint64_t)h->V};
-      cuuint64_t strides[3] = {(cuuint64_t)h->nx * 8, (cuuint64_t)h->nx * h->ny * 8,
-                               (cuuint64_t)h->nx * h->ny * h->nz * 8};
+      cuuint64_t strides[3] = {(cuuint64_t)h->px * 8, (cuuint64_t)h->px * h->ny * 8,
+                               (cuuint64_t)h->px * h->ny * h->nz * 8};
       cuuint32_t box[4] = {(cuuint32_t)fb::ZX, (cuuint32_t)fb::ZY, (cuuint32_t)fb::ZH, 1};
       cuuint32_t es[4] = {1, 1, 1, 1};
       zok = enc(&h->zmaps[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, (void *)h->buf[b], dims,
@@ -272,11 +272,11 @@ bool encode_stage_maps(Handle *h, int hxl) {
                           const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                           const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                           CUtensorMapL2promotion, CUtensorMapFloatOOBfill))fn;
-  const cuuint64_t w = h->fp32 ? 4 : 8, nx = h->nx, ny = h->ny, nz = h->nz;
+  const cuuint64_t w = h->fp32 ? 4 : 8, nx = h->nx, px = h->px, ny = h->ny, nz = h->nz;
   auto one = [&](CUtensorMap *m, void *base, int fields, int bx, int by, int bf) {
     if (!base) return false;
     const cuuint64_t dims[4] = {nx, ny, nz, (cuuint64_t)fields};
-    const cuuint64_t strides[3] = {nx * w, nx * ny * w, nx * ny * nz * w};
+    const cuuint64_t strides[3] = {px * w, px * ny * w, px * ny * nz * w};
     const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, 1, (cuuint32_t)bf};
     const cuuint32_t es[4] = {1, 1, 1, 1};
     return enc(m, h->fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(2 * fb::ZX * fb::ZY)
 // xy: the y and x passes fused; z: the z pass (in -> out, never in place)
 int launch_filter_event(Handle *h, bool xy, const double *in, double *out, cudaStream_t s) {
   FiltArgs<double> F{};
-  F.nx = h->nx; F.ny = h->ny; F.nz = h->nz; F.V = h->V; F.N = h->N;
+  F.nx = h->nx; F.ny = h->ny; F.nz = h->nz; F.px = h->px; F.V = h->V; F.N = h->NP;
   F.periodic = h->periodic ? 1 : 0;
   F.s = xy ? h->P.s_xy : h->P.s_z;
   F.in = in;
@@ -689,7 +689,7 @@ int launch_psr_forcing(Handle *h, const SimDev &S, cudaStream_t s) {
 
 SimDev make_simdev(Handle *h) {
   SimDev S{};
-  S.nx = h->nx; S.ny = h->ny; S.nz = h->nz; S.N = h->N;
+  S.nx = h->nx; S.ny = h->ny; S.nz = h->nz; S.px = h->px; S.N = h->NP;
   S.periodic = h->periodic ? 1 : 0;
   S.magnetic = h->magnetic ? 1 : 0;
   S.bg1d = h->bg1d ? 1 : 0;

@@ -173,7 +173,7 @@ static void filt_launch32(bool xy, const FiltArgs<float> &F, const dim3 &grid, s
 int launch_filter_event32(Handle *h, bool xy, const float *in, const float *carry, float *out,
                           cudaStream_t s) {
   FiltArgs<float> F{};
-  F.nx = h->nx; F.ny = h->ny; F.nz = h->nz; F.V = h->V; F.N = h->N;
+  F.nx = h->nx; F.ny = h->ny; F.nz = h->nz; F.px = h->px; F.V = h->V; F.N = h->NP;
   F.periodic = h->periodic ? 1 : 0;
   F.s = (float)(xy ? h->P.s_xy : h->P.s_z);
   F.in = in;
@@ -300,6 +300,14 @@ int to_float_inv(const double *in, float *out, long long n, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? SPARC_OK : SPARC_ERR_CUDA;
 }
 
+// rows of nx values to rows px apart
+__global__ void k_d2f_rows(const double *__restrict__ in, float *__restrict__ out, int nx, int px,
+                           long long rows) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (long long r = (long long)blockIdx.x * nw + warp; r < rows; r += (long long)gridDim.x * nw)
+    for (int i = lane; i < nx; i += 32) out[r * px + i] = (float)in[r * nx + i];
+}
+
 int to_float(const double *in, float *out, long long n, cudaStream_t s) {
   if (n <= 0) return SPARC_OK;
   unsigned nb = (unsigned)std::min<long long>((n + 255) / 256, 148 * 32);
@@ -310,7 +318,7 @@ int to_float(const double *in, float *out, long long n, cudaStream_t s) {
 // ------------------------------------------------------------- launchers
 Sim32 make_sim32(Handle *h) {
   Sim32 S{};
-  S.nx = h->nx; S.ny = h->ny; S.nz = h->nz; S.N = h->N;
+  S.nx = h->nx; S.ny = h->ny; S.nz = h->nz; S.px = h->px; S.N = h->NP;
   S.periodic = h->periodic ? 1 : 0;
   S.magnetic = h->magnetic ? 1 : 0;
   S.bg1d = h->bg1d ? 1 : 0;
@@ -700,7 +708,7 @@ __global__ void __launch_bounds__(fb::NT)
       continue;
     }
     FiltArgs<float> F{};
-    F.nx = L.S.nx; F.ny = L.S.ny; F.nz = L.S.nz; F.V = L.S.V; F.N = L.S.N;
+    F.nx = L.S.nx; F.ny = L.S.ny; F.nz = L.S.nz; F.px = L.S.px; F.V = L.S.V; F.N = L.S.N;
     F.periodic = L.S.periodic;
     F.s = L.s_xy;
     F.in = L.buf[L.role[0]];
@@ -756,7 +764,7 @@ __global__ void __launch_bounds__(2 * fb::ZX * fb::ZY)
       continue;
     }
     FiltArgs<float> F{};
-    F.nx = L.S.nx; F.ny = L.S.ny; F.nz = L.S.nz; F.V = L.S.V; F.N = L.S.N;
+    F.nx = L.S.nx; F.ny = L.S.ny; F.nz = L.S.nz; F.px = L.S.px; F.V = L.S.V; F.N = L.S.N;
     F.periodic = L.S.periodic;
     F.s = L.s_z;
     F.in = L.buf[L.role[0]];
@@ -905,17 +913,20 @@ int setup32(Handle *h) {
                                        FB_GPX, FB_GPY, FB_GPZ, FB_RHOINV, FB_CBX, FB_CBY,
                                        FB_CBZ, FB_SPONGE, FB_P0, FB_BOX, FB_BOY, FB_BOZ};
   if (h->magnetic) {
-    float *pack = f_up(h, nullptr, PK_COUNT * N, s);
+    float *pack = f_up(h, nullptr, PK_COUNT * h->NP, s);
     if (!pack) return SPARC_ERR_NOMEM;
     h->bg_pack = pack;
-    for (int n = 0; n < PK_COUNT; ++n) h->f_bg[packed[n]] = pack + n * N;
+    for (int n = 0; n < PK_COUNT; ++n) h->f_bg[packed[n]] = pack + n * h->NP;
   }
   for (const Src &q : srcs) {
     const bool one = h->bg1d && q.d1;
     const double *src = one ? q.d1 : q.d3;
     if (!src) continue;
     if (h->f_bg[q.fb]) {
-      if (to_float(src, h->f_bg[q.fb], N, s)) return SPARC_ERR_CUDA;
+      const long long rows = (long long)h->ny * nz;
+      k_d2f_rows<<<(unsigned)std::min<long long>((rows + 7) / 8, 148 * 16), 256, 0, s>>>(
+          src, h->f_bg[q.fb], h->nx, h->px, rows);
+      if (cudaGetLastError() != cudaSuccess) return SPARC_ERR_CUDA;
       continue;
     }
     h->f_bg[q.fb] = f_up(h, src, one ? nz : N, s);
@@ -961,7 +972,7 @@ int setup32(Handle *h) {
     dev_free(h, D.pki);
     D.pa = D.pb = D.pk = D.pki = nullptr;
   }
-  h->tma = h->magnetic && !(h->nx & 3) && h->allow_tma32 &&
+  h->tma = h->magnetic && !(h->px & 3) && h->allow_tma32 &&
            encode_stage_maps(h, MhdBuf<float, true>::HXL);
   return SPARC_OK;
 }
