@@ -115,10 +115,21 @@ struct Rnd32 {
   double timestep, cad;
 };
 
+// tensor maps, all of 4-D views: the state buffers (nx, ny, nz, V) in boxes
+// of one field's 32 x 8 own points [0..2], of all fields' [3..5] and of seven
+// fields' halo planes [6..8]; the packed background (nx, ny, nz, 18) in boxes
+// of 13 arrays' own points [9], of one's [10] and of the three B0 halo
+// planes [11] and of the three B0 own points [12]
+struct TmaSet {
+  CUtensorMap m[13];
+};
+
 // One simulation of a batch, as the batched kernels read it.  Buffer roles,
 // the steps left and the completion counter live here and are advanced on
 // the device, so a captured step stays valid while simulations come and go.
 struct Slot32 {
+  TmaSet T;                    // tensor maps of an MHD member (has_maps)
+  int has_maps;
   SimT<float> S;
   Psr32 psr;
   float *buf[3];
@@ -229,6 +240,7 @@ struct Handle {
   // half spectrum, the spectrum and the three velocity terms
   bool damping = false, fft_plans = false;
   int fft_fwd = 0, fft_inv = 0;  // cufftHandle
+  int damp_fields = 3;           // velocities per transform
   double *d_damp = nullptr, *d_term = nullptr;
   double2 *d_spec = nullptr;
 
@@ -254,7 +266,7 @@ struct Handle {
   // stage kernels (as TmaSet of mhd_body.cuh)
   void *bg_pack = nullptr;
   bool tma = false;
-  CUtensorMap tmaps[13];
+  TmaSet tmaps;
   // FILTER_VARS xy pass (non-periodic FP64 grids, nx even): the state
   // buffers in 44x44x1 boxes
   bool ftma = false;

@@ -26,6 +26,15 @@ enum { F_FIRST = 0, F_MID = 1, F_LAST = 2 };
 template <class R>
 __device__ __forceinline__ R dcoef(int r, int m);
 
+// The two mbarriers of a block's layer buffers, initialised once per launch
+// (a block that takes several items keeps the parity of their next phase in
+// mhd_body's `phase`); by one thread, before a block barrier.
+__device__ __forceinline__ void mhd_bars_init(unsigned long long *bar) {
+  mbar_init_t(&bar[0]);
+  mbar_init_t(&bar[1]);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
 // geometry of the MHD stage tile (precision independent)
 namespace mg {
 // The KE norm is summed over segments of KSEG layers of a tile, so that it
@@ -73,15 +82,6 @@ struct MhdBuf {
   static constexpr size_t smem_bytes(int zext) {
     return SMEM + (sizeof(R) == 4 ? (size_t)(zext + 16) * 16 * sizeof(R) : 0);
   }
-};
-
-// tensor maps, all of 4-D views: the state buffers (nx, ny, nz, V) in boxes
-// of one field's 32 x 8 own points [0..2], of all fields' [3..5] and of seven
-// fields' halo planes [6..8]; the packed background (nx, ny, nz, 18) in boxes
-// of 13 arrays' own points [9], of one's [10] and of the three B0 halo
-// planes [11] and of the three B0 own points [12]
-struct TmaSet {
-  CUtensorMap m[13];
 };
 
 template <class R>
@@ -450,15 +450,16 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
                                          const R *__restrict__ tin,
                                          R *__restrict__ so, R beta, R bnext,
                                          int x0, int y0, int k0, int k1, int mt, int ma,
-                                         double &ke, double &mr, double &mp, uint32_t tw = 0,
-                                         double *kseg = nullptr, int kstride = 0) {
+                                         double &ke, double &mr, double &mp,
+                                         unsigned long long *bar, unsigned &phase,
+                                         uint32_t tw = 0, double *kseg = nullptr,
+                                         int kstride = 0) {
   static_assert(!TW || sizeof(R) == 8, "TMEM windows of FP64 values");
   using namespace mg;
   static_assert(TMA || !TH, "halo boxes come with the own-point boxes");
   using MB = MhdBuf<R, TH>;
   constexpr int BUF = MB::BUF, HXL = MB::HXL, XOFF = MB::XOFF, HSL = MB::HSL, HB = MB::HB;
   constexpr bool SCALED = sizeof(R) == 4;
-  __shared__ unsigned long long bar[2];
   const int tx = threadIdx.x, ty = threadIdx.y, role = threadIdx.z;
   const int tid = (role * TY + ty) * TX + tx, cid = ty * TX + tx;
   const int nx = S.nx, ny = S.ny, nz = S.nz;
@@ -534,11 +535,6 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
     }
     if (isx) cxb[q0] = base;
     else cyb[q0] = base;
-  }
-  if (TMA && tid == 0) {
-    mbar_init_t(&bar[0]);
-    mbar_init_t(&bar[1]);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   auto O = [&](int b, int slot) -> R { return smem[b * BUF + slot * NC + cid]; };
@@ -764,7 +760,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       tm_st_window(tm_window(tw, 2), w2);
     }
   }
-  unsigned phase = 0;
+  int bfail = 0;  // buffer of the layer whose wait gave up
   int rr = 0;  // TW: ring position of the windows (logical value 0 in slot rr)
   bool ok = true;
   const R dt = (R)S.deltat;
@@ -873,7 +869,11 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
     }
     if (TMA && !TH && tid == 0) mine = mbar_wait_t(&bar[b], (phase >> b) & 1u, S.err);
     phase ^= 1u << b;
-    if (!__syncthreads_and(mine)) { ok = false; break; }
+    if (!__syncthreads_and(mine)) {
+      ok = false;
+      bfail = b;
+      break;
+    }
     if (k + 1 < k1) issue(k + 1, b ^ 1);
     if (act && k + 1 < k1 && k + 1 <= nz - 6) head_load(k + 6);
     if constexpr (!TW) {
@@ -1111,10 +1111,8 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
   }
   if (!ok) {
     asm volatile("cp.async.wait_all;\n" ::: "memory");
-    if (TMA && tid == 0) {
-      mbar_wait_t(&bar[0], phase & 1u, S.err);
-      mbar_wait_t(&bar[1], (phase >> 1) & 1u, S.err);
-    }
+    // the copies of the layer given up, the only ones in flight, land first
+    if (TMA && tid == 0) mbar_wait_t(&bar[bfail], ((phase >> bfail) & 1u) ^ 1u, S.err);
     return false;
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");

@@ -287,14 +287,14 @@ bool encode_stage_maps(Handle *h, int hxl) {
   bool ok = true;
   for (int b = 0; b < 3; ++b) {
     void *st = h->fp32 ? (void *)h->fbuf[b] : (void *)h->buf[b];
-    ok = ok && one(&h->tmaps[b], st, h->V, mg::TX, mg::TY, 1) &&
-         one(&h->tmaps[3 + b], st, h->V, mg::TX, mg::TY, 8) &&
-         one(&h->tmaps[6 + b], st, h->V, hxl, mg::HY, 7);
+    ok = ok && one(&h->tmaps.m[b], st, h->V, mg::TX, mg::TY, 1) &&
+         one(&h->tmaps.m[3 + b], st, h->V, mg::TX, mg::TY, 8) &&
+         one(&h->tmaps.m[6 + b], st, h->V, hxl, mg::HY, 7);
   }
-  return ok && one(&h->tmaps[9], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 13) &&
-         one(&h->tmaps[10], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 1) &&
-         one(&h->tmaps[11], h->bg_pack, PK_COUNT, hxl, mg::HY, 3) &&
-         one(&h->tmaps[12], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 3);
+  return ok && one(&h->tmaps.m[9], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 13) &&
+         one(&h->tmaps.m[10], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 1) &&
+         one(&h->tmaps.m[11], h->bg_pack, PK_COUNT, hxl, mg::HY, 3) &&
+         one(&h->tmaps.m[12], h->bg_pack, PK_COUNT, mg::TX, mg::TY, 3);
 }
 
 // ------------------------- MP_MHD_3D, shared-body stage kernel
@@ -320,9 +320,15 @@ __global__ void __launch_bounds__(mg::NT, 1)
   double *smem = (double *)(((size_t)smem_raw64 + 127) & ~(size_t)127);
   __shared__ uint32_t s_tmem;
   __shared__ int s_w;
+  __shared__ unsigned long long bar[2];
+  unsigned phase = 0;
   const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
   const int warp = tid / 32;
-  if (warp == 0) tm_alloc_all(&s_tmem);
+  if (warp == 0) {
+    if (TMA && tid == 0) mhd_bars_init(bar);
+    __syncwarp();
+    tm_alloc_all(&s_tmem);
+  }
   tm_fence_before();
   __syncthreads();
   tm_fence_after();
@@ -357,12 +363,12 @@ __global__ void __launch_bounds__(mg::NT, 1)
     double *kseg = S.kseg + (y0 / mg::TY) * ((S.nx + mg::TX - 1) / mg::TX) + x0 / mg::TX;
     if (in)
       ok = mhd_body<double, MODE, TMA, true, TMA, true>(S, &T, smem, a, tin, so, beta, bnext, x0,
-                                                        y0, k0, k1, mt, ma, ke, mr, mp, tw, kseg,
-                                                        tiles);
+                                                        y0, k0, k1, mt, ma, ke, mr, mp, bar, phase,
+                                                        tw, kseg, tiles);
     else
       ok = mhd_body<double, MODE, TMA, false, TH, true>(S, &T, smem, a, tin, so, beta, bnext, x0,
-                                                        y0, k0, k1, mt, ma, ke, mr, mp, tw, kseg,
-                                                        tiles);
+                                                        y0, k0, k1, mt, ma, ke, mr, mp, bar, phase,
+                                                        tw, kseg, tiles);
     if (!ok) break;
     if (MODE == F_LAST) diag_reduce_mhd(S, mr, mp, w, total, tiles, zchunk);
   }
@@ -429,7 +435,7 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
   if (mt < 0 || ma < 0 || !h->d_wctr64) return SPARC_ERR_INVALID;
   TmaSet T;
   if (tma)
-    std::memcpy(&T, h->tmaps, sizeof(T));
+    T = h->tmaps;
   else
     std::memset(&T, 0, sizeof(T));
   const int nch = (h->nz + h->zchunk - 1) / h->zchunk;

@@ -126,10 +126,14 @@ __global__ void __launch_bounds__(t32::NT, 1)
     if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) atomicExch(S.err, 2);
     return;
   }
+  __shared__ unsigned long long bar[2];
+  unsigned phase = 0;
+  if (TMA && threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) mhd_bars_init(bar);
   double ke = 0.0, mr = 1e300, mp = 1e300;
   const int k0 = blockIdx.z * zchunk;
   if (!mhd_body<float, MODE, TMA, INT, TH>(S, &T, smem, a, tin, so, beta, bnext, x0, y0, k0,
-                                       min(S.nz, k0 + zchunk), mt, ma, ke, mr, mp, 0,
+                                       min(S.nz, k0 + zchunk), mt, ma, ke, mr, mp, bar,
+                                       phase, 0,
                                        S.kseg + tx_ + (long long)gx * ty_, gx * gy))
     return;
   if (MODE == F_LAST)
@@ -408,7 +412,7 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
     if (mt < 0 || ma < 0) return SPARC_ERR_INVALID;
     TmaSet T;
     if (h->tma)
-      std::memcpy(&T, h->tmaps, sizeof(T));
+      T = h->tmaps;
     else
       std::memset(&T, 0, sizeof(T));
     dim3 blk(TX, TY, 2);
@@ -552,11 +556,12 @@ __global__ void k_batch_begin(Slot32 *slots, int n) {
     slots[q].active = slots[q].remaining > 0 ? 1 : 0;
 }
 
-// PART 0: the interior MHD items (a prefix of the list, branch-free body);
-// PART 1: the rest (MHD tiles at edges/CPML, quiet tiles); PART 2: the whole
-// list in one launch (interior items first, then the rest, so no launch
-// boundary separates the two parts).
-template <int MODE, int PART>
+// The whole work-list in one launch: first the interior MHD items (a prefix
+// of the list, counts[3] long), then MHD tiles at edges/CPML and quiet tiles.
+// MHD members with tensor maps take the single path's bodies; the edge tiles
+// of periodic ones, whose halos wrap, and members without maps the cp.async
+// one.
+template <int MODE>
 __global__ void __launch_bounds__(BT, 1)
     k_batch_stage(Slot32 *__restrict__ slots, const int4 *__restrict__ items,
                   const int *__restrict__ counts, unsigned *wctr, int stage) {
@@ -566,10 +571,13 @@ __global__ void __launch_bounds__(BT, 1)
   float *smem = (float *)(((size_t)smem_raw32 + 127) & ~(size_t)127);
   Sim32 &sS = *reinterpret_cast<Sim32 *>(sS_raw);
   const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
-  const int lo = PART == 1 ? counts[3] : 0, hi = PART == 0 ? counts[3] : counts[0];
-  int cur = -1;
+  __shared__ unsigned long long bar[2];
+  unsigned phase = 0;
+  if (tid == 0) mhd_bars_init(bar);
+  const int hi = counts[0];
+  int cur = -1, maps = 0;
   for (;;) {
-    if (tid == 0) s_w = lo + (int)atomicAdd(wctr, 1u);
+    if (tid == 0) s_w = (int)atomicAdd(wctr, 1u);
     __syncthreads();
     const int w = s_w;
     if (w >= hi) break;
@@ -583,6 +591,13 @@ __global__ void __launch_bounds__(BT, 1)
       const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&L.S);
       for (int q = tid; q < (int)(sizeof(Sim32) / 8); q += BT) sS_raw[q] = src[q];
       cur = it.x;
+      maps = L.has_maps;
+      // the maps lie in global memory, written by a copy before this launch:
+      // each issuing lane acquires them
+      if (maps && (tid & 31) == 0 && tid < 8 * 32)
+        for (int m = 0; m < (int)(sizeof(TmaSet) / sizeof(CUtensorMap)); ++m)
+          asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(&L.T.m[m])
+                       : "memory");
       __syncthreads();
     }
     const int ra = L.role[0], r1 = L.role[1], r2 = L.role[2];
@@ -593,18 +608,24 @@ __global__ void __launch_bounds__(BT, 1)
     const float bnext = (float)(stage < 5 ? L.betas[stage] : sS.deltat);
     const int x0 = it.y, y0 = it.z, k0 = it.w & 0xffff, k1 = it.w >> 16;
     double ke = 0.0, mr = 1e300, mp = 1e300;
-    if (PART == 0 || (PART == 2 && w < counts[3]))
-      mhd_body<float, MODE, false, true, false>(sS, nullptr, smem, a, tin, so, beta, bnext, x0, y0,
-                                         k0, k1, 0, 0, ke, mr, mp);
+    bool ok = true;
+    const int ma = ra, mt = stage == 1 ? ra : ((stage == 2 || stage == 4) ? r1 : r2);
+    if (sS.magnetic && maps && w < counts[3])
+      ok = mhd_body<float, MODE, true, true, true>(sS, &L.T, smem, a, tin, so, beta, bnext, x0,
+                                                   y0, k0, k1, mt, ma, ke, mr, mp, bar, phase);
+    else if (sS.magnetic && maps && !sS.periodic)
+      ok = mhd_body<float, MODE, true, false, true>(sS, &L.T, smem, a, tin, so, beta, bnext, x0,
+                                                    y0, k0, k1, mt, ma, ke, mr, mp, bar, phase);
     else if (sS.magnetic)
-      mhd_body<float, MODE, false, false, false>(sS, nullptr, smem, a, tin, so, beta, bnext, x0, y0,
-                                          k0, k1, 0, 0, ke, mr, mp);
+      ok = mhd_body<float, MODE, false, false, false>(sS, nullptr, smem, a, tin, so, beta, bnext,
+                                                      x0, y0, k0, k1, 0, 0, ke, mr, mp, bar, phase);
     else if (sS.bg1d)
       quiet_body<float, 16, MODE, true, MODE == F_LAST ? 2 : 3>(sS, smem, a, tin, so, beta, bnext, x0, y0, k0, k1,
                                            threadIdx.x, threadIdx.y + 8 * threadIdx.z, ke, mr, mp);
     else
       quiet_body<float, 16, MODE, false, 2>(sS, smem, a, tin, so, beta, bnext, x0, y0, k0, k1,
                                             threadIdx.x, threadIdx.y + 8 * threadIdx.z, ke, mr, mp);
+    if (!ok) return;  // a bounded wait gave up (the member's error flag is up)
     if (MODE == F_LAST) batch_finish_step(L, sS, w, ke, mr, mp, tid);
     __syncthreads();
   }
@@ -821,23 +842,23 @@ size_t batch_stage_smem() { return t32::MB::SMEM; }
 // One persistent launch per RK stage over the whole work-list (MHD items of
 // 32 x 8 columns).
 static void launch_batch_stages(const BatchLaunch &B, cudaStream_t s) {
-  const int sm = (int)t32::MB::smem_bytes(B.zmax);
+  const int sm = (int)MhdBuf<float, true>::smem_bytes(B.zmax);
   static_assert(QuietBuf<float, 16, true, 2, true>::bytes(0) <= t32::MB::smem_bytes(0) &&
                     QuietBuf<float, 16, true, 3, false>::bytes(0) <= t32::MB::smem_bytes(0) &&
                     QuietBuf<float, 16, false, 2, true>::bytes(0) <= t32::MB::smem_bytes(0),
                 "the quiet items' ring fits the buffer of the MHD items");
-  cudaFuncSetAttribute(k_batch_stage<F_FIRST, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  cudaFuncSetAttribute(k_batch_stage<F_MID, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  cudaFuncSetAttribute(k_batch_stage<F_LAST, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  cudaFuncSetAttribute(k_batch_stage<F_FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  cudaFuncSetAttribute(k_batch_stage<F_MID>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  cudaFuncSetAttribute(k_batch_stage<F_LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   const dim3 blk(t32::TX, t32::TY, 2);
   for (int st = 1; st <= 5; ++st) {
     unsigned *c = B.wctr + st;  // work counter of stage st
     if (st == 1)
-      k_batch_stage<F_FIRST, 2><<<B.grid, blk, (size_t)sm, s>>>(B.slots, B.items, B.counts, c, st);
+      k_batch_stage<F_FIRST><<<B.grid, blk, (size_t)sm, s>>>(B.slots, B.items, B.counts, c, st);
     else if (st < 5)
-      k_batch_stage<F_MID, 2><<<B.grid, blk, (size_t)sm, s>>>(B.slots, B.items, B.counts, c, st);
+      k_batch_stage<F_MID><<<B.grid, blk, (size_t)sm, s>>>(B.slots, B.items, B.counts, c, st);
     else
-      k_batch_stage<F_LAST, 2><<<B.grid, blk, (size_t)sm, s>>>(B.slots, B.items, B.counts, c, st);
+      k_batch_stage<F_LAST><<<B.grid, blk, (size_t)sm, s>>>(B.slots, B.items, B.counts, c, st);
   }
 }
 
