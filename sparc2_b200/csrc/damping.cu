@@ -9,8 +9,8 @@
 // real, unnormalised: the 1/(nx*ny) is folded into the rates).  The MPI
 // transposes of the reference only gather whole layers on ranks; the
 // result is the per-layer transform.  Here the transforms are cuFFT plans
-// batched over the nz layers (library FFTs on the handle's stream,
-// capturable in the iteration graph), the rate product is k_damp_mul, and
+// batched over the layers of the three velocities (library FFTs on the
+// handle's stream, capturable in the iteration graph), the rate product is k_damp_mul, and
 // the stage kernels read the three terms where the reference subtracts
 // them (after the boundary zeroing, so the boundary planes get -term).
 #include <cufft.h>
@@ -62,7 +62,15 @@ int damping_setup(Handle *h) {
     }
   }
   h->d_damp = (double *)dev_alloc(h, rates.size() * 8);
-  h->d_spec = (double2 *)dev_alloc(h, (size_t)nh * ny * nz * sizeof(double2));
+  // the three velocities lie one after another: one batch of 3 nz layers
+  // (2 transforms and 1 product per stage where there were 6 and 3; one field
+  // at a time where the spectrum of three does not fit)
+  h->damp_fields = 3;
+  h->d_spec = (double2 *)dev_alloc(h, (size_t)3 * nh * ny * nz * sizeof(double2));
+  if (!h->d_spec) {
+    h->damp_fields = 1;
+    h->d_spec = (double2 *)dev_alloc(h, (size_t)nh * ny * nz * sizeof(double2));
+  }
   h->d_term = (double *)dev_alloc(h, (size_t)3 * h->NP * 8);
   if (!h->d_damp || !h->d_spec || !h->d_term) return SPARC_ERR_NOMEM;
   if (cudaMemcpyAsync(h->d_damp, rates.data(), rates.size() * 8, cudaMemcpyHostToDevice,
@@ -72,10 +80,10 @@ int damping_setup(Handle *h) {
   // (real rows are px values apart, as in the state)
   int n[2] = {ny, nx}, real_e[2] = {ny, h->px}, half_e[2] = {ny, nh};
   if (!fft_ok(h, cufftPlanMany(&h->fft_fwd, 2, n, real_e, 1, h->px * ny, half_e, 1, nh * ny,
-                               CUFFT_D2Z, nz),
+                               CUFFT_D2Z, nz * h->damp_fields),
               "cufftPlanMany (forward)") ||
       !fft_ok(h, cufftPlanMany(&h->fft_inv, 2, n, half_e, 1, nh * ny, real_e, 1, h->px * ny,
-                               CUFFT_Z2D, nz),
+                               CUFFT_Z2D, nz * h->damp_fields),
               "cufftPlanMany (inverse)"))
     return SPARC_ERR_CUDA;
   h->fft_plans = true;
@@ -85,12 +93,12 @@ int damping_setup(Handle *h) {
 // The three damping terms of the velocities of state tin (fields 1..3)
 // into h->d_term, on stream s.
 int damping_enqueue(Handle *h, const double *tin, cudaStream_t s) {
-  const long long nh = (long long)(h->nx / 2 + 1) * h->ny, total = nh * h->nz;
+  const long long nh = (long long)(h->nx / 2 + 1) * h->ny, total = nh * h->nz * h->damp_fields;
   const unsigned blocks = (unsigned)std::min<long long>((total + 255) / 256, 148LL * 16);
   if (!fft_ok(h, cufftSetStream(h->fft_fwd, s), "cufftSetStream") ||
       !fft_ok(h, cufftSetStream(h->fft_inv, s), "cufftSetStream"))
     return SPARC_ERR_CUDA;
-  for (int l = 0; l < 3; ++l) {
+  for (int l = 0; l < 3; l += h->damp_fields) {
     // the forward transform does not write its input (out of place)
     double *in = const_cast<double *>(tin) + (size_t)(l + 1) * h->NP;
     if (!fft_ok(h, cufftExecD2Z(h->fft_fwd, in, (cufftDoubleComplex *)h->d_spec),
