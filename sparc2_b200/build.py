@@ -28,7 +28,7 @@ UNITS = {
     "damping.cu": [],
     "state_io.cu": [],
 }
-HEADERS = ["internal.h", "mhd_body.cuh", "quiet_body.cuh", "random_forcing.cuh", "filter_body.cuh",
+HEADERS = ["internal.h", "mhd_body.cuh", "quiet_body.cuh", "psr_forcing.cuh", "random_forcing.cuh", "filter_body.cuh",
            "tmem_window.cuh", "tma_util.cuh"]
 # host C units (gcc): the .trol reader
 HOST_UNITS = {"sparc_trol.c": ["-O2", "-std=c99", "-Wall", "-fPIC"]}

@@ -893,7 +893,7 @@ int sparc_tune(sparc_handle *h, int64_t first, int steps_per_trial, int64_t *nex
   NOT_IN_BATCH(h);
   if (!h->bg_ready) return fail(h, SPARC_ERR_ORDER, "set the background first");
   cudaSetDevice(h->device);
-  static const int cand[] = {16, 24, 32, 40, 48, 64, 80, 100, 150};
+  static const int cand[] = {12, 16, 24, 32, 40, 48, 64, 80, 100, 150};
   std::vector<int> cs;
   for (int c : cand) {
     const int z = std::min(c, h->nz);

@@ -21,6 +21,7 @@
 
 #include "filter_body.cuh"
 #include "mhd_body.cuh"
+#include "psr_forcing.cuh"
 #include "quiet_body.cuh"
 #include "random_forcing.cuh"
 
@@ -479,10 +480,7 @@ int launch_stage(Handle *h, const SimDev &S, int stage, const double *a,
 }
 
 // ------------------------------------------------------- PULSE = 2 forcing
-// all_modules.f90:592-611 / 644-660 and driver.f90:153 for the layers that
-// carry any pulse: sum over the layer's pulses of
-// T_n(t) * Z_n(k) * X_n(i) * Y_n(j), culled per reference rank block, twice
-// at the run's first iteration, times source_damp * src_scale_beta.
+// The layers that carry any pulse (psr_forcing.cuh).
 struct PsrDev {
   int nx, ny, nz, klo, npulses, nblocks;
   long long init;
@@ -496,38 +494,9 @@ struct PsrDev {
   const long long *iter;
 };
 
-__global__ void k_psr(PsrDev D) {
+__global__ void __launch_bounds__(256) k_psr(PsrDev D) {
   extern __shared__ double sh[];
-  const int k = D.klo + blockIdx.z;
-  const int e0 = D.off[k], e1 = D.off[k + 1], ne = e1 - e0;
-  double *sT = sh;
-  int *sN = (int *)(sh + ne);
-  const long long it = *D.iter;
-  const double t = (double)it * D.timestep;
-  const double passes = (it == D.init) ? 2.0 : 1.0;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  for (int e = tid; e < ne; e += blockDim.x * blockDim.y) {
-    const int n = D.idx[e0 + e];
-    const double amp = D.ptime[3 * n], t0 = D.ptime[3 * n + 1],
-                 t1 = D.ptime[3 * n + 2];
-    double v = amp * sin(2.0 * PI * (t - t1) / t0);
-    v = v * exp(-((t - t1) * (t - t1)) / (2.0 * (D.st * D.st)));
-    sT[e] = v * D.zv[e0 + e] * passes;
-    sN[e] = n;
-  }
-  __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= D.nx || j >= D.ny) return;
-  const int blk = D.colx[i] + D.bx * D.coly[j] + D.bxy * D.colz[k];
-  double f = 0.0;
-  for (int e = 0; e < ne; ++e) {
-    const int n = sN[e];
-    if (!D.mask[(long long)n * D.nblocks + blk]) continue;
-    f = f + sT[e] * (D.px[(long long)n * D.nx + i] * D.py[(long long)n * D.ny + j]);
-  }
-  const long long g = ((long long)k * D.ny + j) * D.nx + i;
-  D.out[((long long)blockIdx.z * D.ny + j) * D.nx + i] = f * D.sd[g] * D.ssb[g];
+  psr_tile<double>(D, sh, D.npulses);
 }
 
 int launch_psr_forcing(Handle *h, const SimDev &S, cudaStream_t s);

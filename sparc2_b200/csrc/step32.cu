@@ -25,6 +25,7 @@
 
 #include "filter_body.cuh"
 #include "mhd_body.cuh"
+#include "psr_forcing.cuh"
 #include "quiet_body.cuh"
 #include "random_forcing.cuh"
 
@@ -211,37 +212,9 @@ int launch_filter_event32(Handle *h, bool xy, const float *in, const float *carr
 // ------------------------------------------------ PULSE = 2, precision form
 // As k_psr of step.cu with an FP32 forcing buffer (the sum over pulses is
 // accumulated in FP32).
-__global__ void k_psr32(Psr32 D) {
+__global__ void __launch_bounds__(256) k_psr32(Psr32 D, int maxp) {
   extern __shared__ float shf[];
-  const int k = D.klo + blockIdx.z;
-  const int e0 = D.off[k], e1 = D.off[k + 1], ne = e1 - e0;
-  float *sT = shf;
-  int *sN = (int *)(shf + ne);
-  const long long it = *D.iter;
-  const double t = (double)it * D.timestep;
-  const double passes = (it == D.init) ? 2.0 : 1.0;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  for (int e = tid; e < ne; e += blockDim.x * blockDim.y) {
-    const int n = D.idx[e0 + e];
-    const double amp = D.ptime[3 * n], t0 = D.ptime[3 * n + 1], t1 = D.ptime[3 * n + 2];
-    double v = amp * sin(2.0 * PI * (t - t1) / t0);
-    v = v * exp(-((t - t1) * (t - t1)) / (2.0 * (D.st * D.st)));
-    sT[e] = (float)(v * D.zv[e0 + e] * passes);
-    sN[e] = n;
-  }
-  __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= D.nx || j >= D.ny) return;
-  const int blk = D.colx[i] + D.bx * D.coly[j] + D.bxy * D.colz[k];
-  float f = 0.f;
-  for (int e = 0; e < ne; ++e) {
-    const int n = sN[e];
-    if (!D.mask[(long long)n * D.nblocks + blk]) continue;
-    f = f + sT[e] * (D.px[(long long)n * D.nx + i] * D.py[(long long)n * D.ny + j]);
-  }
-  const long long g = ((long long)k * D.ny + j) * D.nx + i;
-  D.out[((long long)blockIdx.z * D.ny + j) * D.nx + i] = f * D.sd[g] * D.ssb[g];
+  psr_tile<float>(D, shf, maxp);
 }
 
 Psr32 make_psr32(Handle *h) {
@@ -278,7 +251,7 @@ int launch_psr32(Handle *h, cudaStream_t s) {
   dim3 blk(32, 8);
   dim3 grd((h->nx + 31) / 32, (h->ny + 7) / 8, h->psr_khi - h->psr_klo);
   size_t smem = h->pulses.size() * (sizeof(float) + sizeof(int));
-  k_psr32<<<grd, blk, smem, s>>>(D);
+  k_psr32<<<grd, blk, smem, s>>>(D, (int)h->pulses.size());
   ++h->launches;
   return cudaGetLastError() == cudaSuccess ? SPARC_OK : SPARC_ERR_CUDA;
 }
