@@ -267,11 +267,11 @@ struct Handle {
   void *bg_pack = nullptr;
   bool tma = false;
   TmaSet tmaps;
-  // FILTER_VARS xy pass (non-periodic FP64 grids, nx even): the state
+  // FILTER_VARS xy pass (non-periodic FP64 grids, 16-byte rows): the state
   // buffers in 44x44x1 boxes
   bool ftma = false;
   CUtensorMap fmaps[3];
-  // FILTER_VARS z pass (FP64, nx even): the state buffers as (nx, ny, nz, V)
+  // FILTER_VARS z pass (FP64, 16-byte rows): the state buffers as (nx, ny, nz, V)
   // in 32x4x44x1 boxes
   bool ztma = false;
   CUtensorMap zmaps[3];
@@ -307,8 +307,8 @@ struct Handle {
   float *f_fx = nullptr, *f_fy = nullptr, *f_fz = nullptr;
   float *f_psr = nullptr, *f_px = nullptr, *f_py = nullptr;
   float *f_sd = nullptr, *f_ssb = nullptr;
-  bool allow_tma32 = true;   // FP32 MHD own-point loads by TMA (nx % 4 == 0)
-  bool allow_tma64 = true;   // FP64 MHD own-point loads by TMA (nx even)
+  bool allow_tma32 = true;   // FP32 MHD copies by TMA
+  bool allow_tma64 = true;   // FP64 MHD copies by TMA
 
   // member of a batch (sparc_batch_add): the batch owns the buffer roles,
   // the iteration and the stream order until sparc_batch_remove

@@ -3,12 +3,23 @@
 // plain form (R = double, step.cu) and the precision form (R = float,
 // step32.cu, with depth-scaled state and a compensated final update).
 //
-// Two roles per column (threadIdx.z): role 0 computes the momentum
-// equations (z windows vz, p, bx), role 1 continuity, pressure and
-// induction (z windows flux1, flux2, by); d(vz)/dz and d(by)/dz cross over
-// through shared memory.  A CTA owns a 32x8 column tile and marches a chunk
-// of z layers; the layer's halo planes and own-point arrays are copied into
-// a double-buffered shared tile one layer ahead.
+// Two roles per column: role 0 (warps 0..7) computes the momentum equations
+// (z windows p, bx, by), role 1 (warps 8..15) continuity, pressure and
+// induction (z windows flux1, flux2, vz), so that no derivative crosses
+// between them.  A CTA owns a 32x8 column tile and marches a chunk of z
+// layers; the layer's halo planes and own-point arrays are copied into a
+// double-buffered shared tile one layer ahead, by five to seven tensor copies
+// where the tile's halos do not wrap.
+//
+// What bounds it: one 512-thread block per SM (registers, and 226 KB of
+// shared memory in FP64) goes through the phases of a layer in step.  Of an
+// interior FP64 layer's 6,100 cycles the x/y stencils take 2,000 (60 shared
+// loads of 8 bytes per thread, the shared memory's rate), the z windows
+// 1,100, the update 1,100, the fluxes and the wait for the copies 550, the
+// layer barrier 400, heads and copies 800; an edge tile's 9,600 have 1,400
+// for CPML and 2,700 for one-sided stencils.  Measured on 256x256x300, per
+// iteration, before and after the present layout of roles, copies and heads:
+// FP64 12.58 -> 10.4 ms, FP32 10.29 -> 7.6 ms.
 //
 // Each translation unit that includes this header defines
 // dcoef<R>(row, m): its constant table of the derivative rows
@@ -432,18 +443,21 @@ inline void mhd_interior_rect(int nx, int ny, const int np[4], int &ix0, int &ix
 // x/y derivatives are the centred stencil with no branch.  Returns false
 // when a bounded wait gave up.
 //
-// Per layer: every thread waits for its own halo copies, turns the B0 halo
-// values it copied into the fluxes v x B0 in place, then one barrier makes
-// the layer visible; the copies of the next layer are issued after that
-// barrier (the buffer they overwrite was last read before it).  A named
-// barrier of the two warps that share rows ty (role 0 warp ty, role 1 warp
-// 8 + ty) exchanges d(vz)/dz and d(by)/dz: nothing else crosses warps
-// until the next layer's barrier.
+// Per layer: every thread waits for the layer's copies (its own ones without
+// TH), turns the B0 values of its halo positions into the fluxes v x B0 in
+// place, then one barrier makes the layer visible; the copies of the next
+// layer are issued after that barrier (the buffer they overwrite was last
+// read before it), and the values of the next window heads loaded.  Nothing
+// else crosses warps until the next layer's barrier, except |v_new|^2 of the
+// last stage (the two warps of a row).
 //
 // TW (FP64): the z windows live in tensor memory between layers
 // (tmem_window.cuh; tw is this warp's window address, the caller allocates
-// and frees): each layer loads them, shifts in the new head, stores them
-// back and forms the z derivatives, so they hold registers only then.
+// and frees): each layer loads them, stores the new head and forms the z
+// derivatives, so they hold registers only then.  bar, phase: the two
+// barriers of the layer buffers and the parity of their next phases
+// (mhd_bars_init).  kseg: where the KE sums of the tile's segments go (stride
+// kstride per part), or null (ke accumulates).
 template <class R, int MODE, bool TMA, bool INT, bool TH, bool TW = false>
 __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *smem,
                                          const R *__restrict__ a,

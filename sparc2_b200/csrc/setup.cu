@@ -357,13 +357,18 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
   if (!h->d_stretch) return SPARC_ERR_NOMEM;
 
   // ------------------------------------------------ 3-D arrays (FP64)
-  // MHD in the plain form: the arrays of the stage kernels in one allocation
+  // MHD in the plain form: the arrays of the stage kernels in one allocation.
+  // Where its rows are padded, they are set up in the state buffers (24 fields,
+  // cleared afterwards) and copied into it at the end.
   double *pack = nullptr;
-  if (h->magnetic && !h->fp32 && h->px == nx) {
-    h->bg_pack = pack = up(h, nullptr, PK_COUNT * N);
+  if (h->magnetic && !h->fp32) {
+    h->bg_pack = pack = up(h, nullptr, PK_COUNT * h->NP);
     if (!pack) return SPARC_ERR_NOMEM;
   }
-  auto bga = [&](int n) -> double * { return pack ? pack + n * N : up(h, nullptr, N); };
+  auto bga = [&](int n) -> double * {
+    if (!pack) return up(h, nullptr, N);
+    return h->px == nx ? pack + n * N : h->buf[n / 8] + (long long)(n % 8) * N;
+  };
   double *rho0 = h->rho0 = bga(PK_RHO0);
   double *p0 = h->p0 = bga(PK_P0);
   double *c2 = h->c2 = up(h, nullptr, N);
@@ -774,20 +779,14 @@ int setup_background(Handle *h, const double *rho0_in, const double *pre0_in,
     each(n, s, [=] __device__(long long t) { ki[t] = 1.0 / pk[t]; });
     F.pki = ki;
   }
-  // plain-form MHD with padded rows: the arrays set up so far, packed
-  if (h->magnetic && !h->fp32 && !pack) {
+  // plain-form MHD with padded rows: out of the state buffers
+  if (pack && h->px != nx) {
     double **arr[PK_COUNT] = {&h->red, &h->rho0, &h->grx, &h->gry, &h->grz, &h->c2rho0,
                               &h->gpx, &h->gpy, &h->gpz, &h->rhoinv, &h->cbx, &h->cby,
                               &h->cbz, &h->sponge, &h->p0, &h->box, &h->boy, &h->boz};
-    pack = up(h, nullptr, PK_COUNT * h->NP);
-    if (!pack) return SPARC_ERR_NOMEM;
-    h->bg_pack = pack;
-    for (int n = 0; n < PK_COUNT; ++n)
+    for (int n = 0; n < PK_COUNT; ++n) {
       if (repitch(*arr[n], nx, pack + n * h->NP, h->px, nx, (long long)ny * nz, s))
         return SPARC_ERR_CUDA;
-    CK(cudaStreamSynchronize(s));
-    for (int n = 0; n < PK_COUNT; ++n) {
-      dev_free(h, *arr[n]);
       *arr[n] = pack + n * h->NP;
     }
   }

@@ -93,11 +93,10 @@ __global__ void __launch_bounds__(qg::TX *Quiet32<MODE, BG1D>::TY, Quiet32<MODE,
 // -------------------------------------------- MP_MHD_3D, precision form
 // The two-role body of mhd_body.cuh in FP32 with depth scaling (field
 // scales: 0 rho, 1-3 v, 4 p, 5-7 b), one row of columns per thread: a CTA
-// of 512 threads owns a 32 x 8 column tile.  Own-point arrays of a layer
-// arrive by TMA (32x8 FP32 boxes), halos by cp.async; one CTA per SM.  (Two
-// rows per thread measured 30 % slower on the 256x256x300 flux tube: the
-// register spills of the doubled windows land in L2, the shared-memory
-// carve-out leaving little L1.)
+// of 512 threads owns a 32 x 8 column tile; one CTA per SM.  (Two rows per
+// thread measured 30 % slower on the 256x256x300 flux tube: the register
+// spills of the doubled windows land in L2, the shared-memory carve-out
+// leaving little L1.)
 
 namespace t32 {
 using namespace mg;
