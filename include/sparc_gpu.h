@@ -175,9 +175,10 @@ int sparc_run(sparc_handle *h, int64_t first, int64_t count);
 
 /* z extent of the stage kernels' work items (a work item is a 32 x 8
  * column tile over zchunk layers; each item pays 10 layers of z-window
- * warm-up).  No counterpart in the reference.  11 <= zchunk (clamped to
- * nz); set up from the grid size, changed by sparc_set_zchunk or
- * sparc_tune.  Results do not depend on it. */
+ * warm-up).  No counterpart in the reference.  Set up from the grid size
+ * (on small grids below 11), changed by sparc_set_zchunk (the set-up extent,
+ * or 11 <= zchunk, clamped to nz) or sparc_tune.  Quiet stages take at most 32
+ * layers per block.  Results do not depend on it. */
 int sparc_set_zchunk(sparc_handle *h, int zchunk);
 int sparc_get_zchunk(const sparc_handle *h, int *zchunk);
 

@@ -866,7 +866,8 @@ static int set_zchunk(Handle *h, int zc) {
 }
 
 int sparc_set_zchunk(sparc_handle *h, int zchunk) {
-  if (!h || zchunk < 11) return SPARC_ERR_INVALID;
+  // (the set-up extent, which may be shorter, can be set again)
+  if (!h || (zchunk < 11 && zchunk != h->zchunk0)) return SPARC_ERR_INVALID;
   NOT_IN_BATCH(h);
   cudaSetDevice(h->device);
   CK(h, cudaStreamSynchronize(h->stream));  // graphs in flight finish first

@@ -287,10 +287,11 @@ struct Handle {
   int2 *d_gen = nullptr;
   int ngen = 0, gix0 = 0, giy0 = 0, gnix = 0, gniy = 0, pgrid = 0;
   unsigned *d_wctr64 = nullptr;
-  int partials_blocks = 0;  // blocks the partials hold: any z chunk >= 11
+  int partials_blocks = 0;  // blocks the partials hold: the set-up extent, any >= 11
 
   // layers per z chunk of the stage work items (tiles of 32 x 8 columns)
   int zchunk = 32;
+  int zchunk0 = 32;  // as set up
 
   // precision form (SPARC_FP32): FP32 state in fbuf (roles ra/rf1/rf2 as
   // for buf), the compensated-sum carry of the state, depth scales

@@ -161,7 +161,7 @@ int stage_geometry(Handle *h) {
     const int v = std::atoi(kv);
     if (v >= 4) zc = std::min(v, h->nz);
   }
-  h->zchunk = zc;
+  h->zchunk = h->zchunk0 = zc;
   h->max_stage_blocks = (int)(tiles * ((h->nz + zc - 1) / zc));
   const int zmin = std::min(zc, 11);
   h->partials_blocks = (int)(tiles * ((h->nz + zmin - 1) / zmin));

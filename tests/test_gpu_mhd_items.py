@@ -49,6 +49,18 @@ def test_batch_items_of_odd_layers(sizes):
             assert cases.rel_l2(a[l], want[l]) <= 1e-6
 
 
+def test_set_up_extent_can_be_set_again():
+    s = sim_of(40, 40, 48, abi.SPARC_FP64)
+    zc = s.zchunk
+    assert 4 <= zc <= 48
+    s.set_zchunk(24)
+    s.set_zchunk(zc)
+    assert s.zchunk == zc
+    if zc != 5:
+        with pytest.raises(abi.SparcError):
+            s.set_zchunk(5)
+
+
 def test_persistent_items_of_odd_layers():
     # 4 x 20 tiles: about 400 items at 11 layers, 240 at 17, on 148 blocks
     got = []
