@@ -46,6 +46,14 @@ __device__ __forceinline__ void mhd_bars_init(unsigned long long *bar) {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+// `phase` after a layer in buffer b.  Only a body with tensor copies arrives on
+// the barriers; one without leaves them, and so their parities, as they are
+// (a batch runs both kinds of items in one block).
+template <bool TMA>
+__host__ __device__ __forceinline__ unsigned mhd_next_phase(unsigned phase, int b) {
+  return TMA ? phase ^ (1u << b) : phase;
+}
+
 // geometry of the MHD stage tile (precision independent)
 namespace mg {
 // The KE norm is summed over segments of KSEG layers of a tile, so that it
@@ -882,7 +890,7 @@ __device__ __forceinline__ bool mhd_body(const SimT<R> &S, const TmaSet *T, R *s
       flux(b, hs1, u0, u1, u2);
     }
     if (TMA && !TH && tid == 0) mine = mbar_wait_t(&bar[b], (phase >> b) & 1u, S.err);
-    phase ^= 1u << b;
+    phase = mhd_next_phase<TMA>(phase, b);
     if (!__syncthreads_and(mine)) {
       ok = false;
       bfail = b;
