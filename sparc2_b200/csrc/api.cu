@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "tma_util.cuh"
 
 namespace sparc {
 
@@ -310,30 +311,15 @@ static Handle::GraphEntry *graph_for(Handle *h, int fk) {
 }
 
 // Failure injection: one thread waits on an mbarrier that expects one
-// arrival which never comes; the bounded wait gives up after `polls` polls
-// or 10 ms of the global timer, whichever comes first, and raises the error
-// flag, as a stage kernel's gave-up wait does.
+// arrival which never comes; the stage kernels' bounded wait gives up after
+// `polls` polls or 10 ms of the global timer, whichever comes first, and raises
+// the error flag.
 __global__ void k_wait_probe(int *err, long long polls) {
   __shared__ unsigned long long bar;
   if (threadIdx.x != 0) return;
-  const unsigned a = (unsigned)__cvta_generic_to_shared(&bar);
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a) : "memory");
+  mbar_init_t(&bar);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  unsigned long long t0, t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  for (long long n = 0; n < polls; ++n) {
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    if (t - t0 > 10000000ull) break;
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(a), "r"(0u)
-        : "memory");
-    if (ok) return;
-  }
-  atomicExch(err, 1);
+  mbar_wait_t(&bar, 0u, err, (unsigned)polls, 10000000u);
 }
 
 }  // namespace sparc

@@ -63,7 +63,6 @@ constexpr int KSEG = 4;
 constexpr int TX = 32, TY = 8, NC = TX * TY, NT = 2 * NC;
 constexpr int HX = TX + 10, HY = TY + 10, HS = HX * HY;
 constexpr int NH = 10, NO = 24;
-constexpr long long WAIT_LIMIT = kMbarWaitLimit;
 // own-point slots: stage rho, a[0..7], 14 background arrays, p0
 constexpr int O_RHO = 0, O_A = 1, O_BG = 9, O_P0 = 23;
 // (the order of the packed background arrays, internal.h)

@@ -8,8 +8,12 @@
 
 namespace sparc {
 
-// polls of an mbarrier before a wait gives up and raises the error flag
-constexpr long long kMbarWaitLimit = 1LL << 26;
+// A wait on an mbarrier gives up and raises the error flag after kMbarWaitNs
+// of the global timer (copies land within microseconds; another context's time
+// slices may come in between), or after kMbarWaitLimit polls where that timer
+// stands still.  Polls alone are no bound on time: each may itself suspend.
+constexpr unsigned kMbarWaitLimit = 1u << 26;
+constexpr unsigned kMbarWaitNs = 1000000000u;
 
 __device__ __forceinline__ unsigned sm_addr_t(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
@@ -48,20 +52,46 @@ __device__ __forceinline__ void tma4d_l2(const CUtensorMap *map, int x, int y, i
                "r"(x), "r"(y), "r"(z), "r"(w)
                : "memory");
 }
-// bounded wait: gives up after kMbarWaitLimit polls and raises the error flag
-__device__ __forceinline__ bool mbar_wait_t(unsigned long long *bar, unsigned parity, int *err) {
-  for (long long n = 0; n < kMbarWaitLimit; ++n) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(sm_addr_t(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
+// Polls `done` until it is true, at most `polls` times and about `ns` of the
+// clock `now` (32 bits of nanoseconds, read every 64 polls: waits that end soon
+// do not read it).
+template <class Done, class Now>
+__host__ __device__ __forceinline__ bool bounded_polls(Done done, Now now, unsigned polls,
+                                                       unsigned ns) {
+  unsigned t0 = 0;
+  for (unsigned n = 0; n < polls; ++n) {
+    if (done()) return true;
+    if ((n & 63u) == 63u) {
+      const unsigned t = now();
+      if (n == 63u) t0 = t;
+      else if (t - t0 > ns) return false;
+    }
   }
-  atomicExch(err, 1);
   return false;
+}
+// bounded wait: the error flag where it gave up
+__device__ __forceinline__ bool mbar_wait_t(unsigned long long *bar, unsigned parity, int *err,
+                                            unsigned polls = kMbarWaitLimit,
+                                            unsigned ns = kMbarWaitNs) {
+  const bool ok = bounded_polls(
+      [&] {
+        unsigned r;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(r)
+            : "r"(sm_addr_t(bar)), "r"(parity)
+            : "memory");
+        return r != 0;
+      },
+      [] {
+        unsigned t;
+        asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+        return t;
+      },
+      polls, ns);
+  if (!ok) atomicExch(err, 1);
+  return ok;
 }
 
 }  // namespace sparc
