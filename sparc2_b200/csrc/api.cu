@@ -551,6 +551,8 @@ int sparc_set_background(sparc_handle *h, const double *rho0,
     r = encode_tensor_maps(h);
     if (r) return r;
   }
+  if (h->fp32 ? stage_limits32(h) : stage_limits(h))
+    return fail(h, SPARC_ERR_CUDA, "shared memory of the stage kernels");
   r = zero_state(h);
   if (r) return r;
   h->bg_ready = true;

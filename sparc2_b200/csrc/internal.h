@@ -350,6 +350,25 @@ int launch_psr_forcing(Handle *h, const SimDev &S, cudaStream_t s);
 int launch_random_forcing(Handle *h, cudaStream_t s);
 int launch_filter_event(Handle *h, bool xy, const double *in, double *out, cudaStream_t s);
 int stage_geometry(Handle *h);
+
+// Raises a kernel's limit of dynamic shared memory to all that the device gives
+// a block beside the kernel's static part.  The limit belongs to the kernel, not
+// to a handle: set to what each launch takes, as it was, a handle of a shorter z
+// extent on one thread lowered it between another's setting and launch, which was
+// then refused.  Set once per handle (or batch capture), before the launches.
+template <class K>
+int allow_smem(K *kernel) {
+  cudaFuncAttributes at;
+  int dev = 0, cap = 0;
+  const bool ok =
+      cudaFuncGetAttributes(&at, kernel) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           cap - (int)at.sharedSizeBytes) == cudaSuccess;
+  return ok ? SPARC_OK : SPARC_ERR_CUDA;
+}
+int stage_limits(Handle *h);
+int stage_limits32(Handle *h);
 int encode_tensor_maps(Handle *h);
 bool encode_stage_maps(Handle *h, int hxl);
 int repitch(const double *src, int sp, double *dst, int dp, int nx, long long rows,

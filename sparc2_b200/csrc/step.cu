@@ -177,11 +177,7 @@ static int launch_quiet(Handle *h, const SimDev &S, int stage, const double *a,
   const double bnext = stage < 5 ? h->betas[stage] : h->deltat;
   const int mode = stage == 1 ? FIRST : (stage == 5 ? LAST : MID);
 #define QL(M, B)                                                                          \
-  do {                                                                                    \
-    const int sm = (int)Quiet64<B>::Buf::bytes(zc);                                       \
-    cudaFuncSetAttribute(k_quiet64<M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm); \
-    k_quiet64<M, B><<<grd, blk, sm, s>>>(S, a, tin, so, beta, bnext, zc);                 \
-  } while (0)
+  k_quiet64<M, B><<<grd, blk, Quiet64<B>::Buf::bytes(zc), s>>>(S, a, tin, so, beta, bnext, zc)
   if (S.bg1d) {
     if (mode == FIRST) QL(F_FIRST, true);
     else if (mode == MID) QL(F_MID, true);
@@ -446,12 +442,8 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
   unsigned *ctr = h->d_wctr64 + (stage - 1);
   const dim3 blk(mg::TX, mg::TY, 2);
 #define MP64(M, U, H)                                                                        \
-  do {                                                                                       \
-    cudaFuncSetAttribute(k_mhd64p<M, U, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
-                         (int)sm);                                                           \
-    k_mhd64p<M, U, H><<<grid, blk, sm, s>>>(S, T, a, tin, so, beta, bnext, h->zchunk, mt, ma, h->gix0,   \
-                                        h->giy0, h->gnix, nint, h->ngen, h->d_gen, ctr);     \
-  } while (0)
+  k_mhd64p<M, U, H><<<grid, blk, sm, s>>>(S, T, a, tin, so, beta, bnext, h->zchunk, mt, ma,   \
+                                      h->gix0, h->giy0, h->gnix, nint, h->ngen, h->d_gen, ctr)
   if (th) {
     if (mode == FIRST) MP64(F_FIRST, true, true);
     else if (mode == MID) MP64(F_MID, true, true);
@@ -467,6 +459,27 @@ static int launch_mhd64p(Handle *h, const SimDev &S, int stage, const double *a,
   }
 #undef MP64
   return SPARC_OK;
+}
+
+// The stage kernels that the handle launches, allowed their shared memory
+// (after encode_tensor_maps).
+int stage_limits(Handle *h) {
+  int r = SPARC_OK;
+#define LIM(K, ...) \
+  r |= allow_smem(K<F_FIRST, __VA_ARGS__>) | allow_smem(K<F_MID, __VA_ARGS__>) | \
+       allow_smem(K<F_LAST, __VA_ARGS__>)
+  if (!h->magnetic) {
+    if (h->bg1d) LIM(k_quiet64, true);
+    else LIM(k_quiet64, false);
+  } else if (h->tma && !h->periodic) {
+    LIM(k_mhd64p, true, true);
+  } else if (h->tma) {
+    LIM(k_mhd64p, true, false);
+  } else {
+    LIM(k_mhd64p, false, false);
+  }
+#undef LIM
+  return r ? SPARC_ERR_CUDA : SPARC_OK;
 }
 
 int launch_stage(Handle *h, const SimDev &S, int stage, const double *a,

@@ -352,11 +352,7 @@ static void launch_quiet32(Handle *h, const Sim32 &S, int mode, const float *a,
   const dim3 blk(qg::TX, 8);
   const dim3 grd((h->nx + qg::TX - 1) / qg::TX, (h->ny + 7) / 8, (h->nz + zc - 1) / zc);
 #define QL32(M, B)                                                                        \
-  do {                                                                                    \
-    const int sm = (int)Quiet32<M, B>::Buf::bytes(zc);                                     \
-    cudaFuncSetAttribute(k_quiet32<M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm); \
-    k_quiet32<M, B><<<grd, blk, sm, s>>>(S, a, tin, so, beta, bnext, zc);                 \
-  } while (0)
+  k_quiet32<M, B><<<grd, blk, Quiet32<M, B>::Buf::bytes(zc), s>>>(S, a, tin, so, beta, bnext, zc)
   if (S.bg1d) {
     if (mode == F_FIRST) QL32(F_FIRST, true);
     else if (mode == F_MID) QL32(F_MID, true);
@@ -367,6 +363,28 @@ static void launch_quiet32(Handle *h, const Sim32 &S, int mode, const float *a,
     else QL32(F_LAST, false);
   }
 #undef QL32
+}
+
+// The stage kernels that the handle launches, allowed their shared memory
+// (after the tensor maps).
+int stage_limits32(Handle *h) {
+  int r = SPARC_OK;
+#define LIM(K, ...) \
+  r |= allow_smem(K<F_FIRST, __VA_ARGS__>) | allow_smem(K<F_MID, __VA_ARGS__>) | \
+       allow_smem(K<F_LAST, __VA_ARGS__>)
+  if (!h->magnetic) {
+    if (h->bg1d) LIM(k_quiet32, true);
+    else LIM(k_quiet32, false);
+  } else if (h->tma) {
+    LIM(k_mhd32, true, true, true);
+    if (h->periodic) LIM(k_mhd32, true, false, false);
+    else LIM(k_mhd32, true, false, true);
+  } else {
+    LIM(k_mhd32, false, true, false);
+    LIM(k_mhd32, false, false, false);
+  }
+#undef LIM
+  return r ? SPARC_ERR_CUDA : SPARC_OK;
 }
 
 int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
@@ -405,8 +423,6 @@ int launch_stage32(Handle *h, const Sim32 &S, int stage, const float *a,
     const int smz = th ? smi : (int)MB::smem_bytes(h->zchunk);
 #define ML32(M, U, H)                                                                       \
   do {                                                                                      \
-    cudaFuncSetAttribute(k_mhd32<M, U, true, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi); \
-    cudaFuncSetAttribute(k_mhd32<M, U, false, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, smz); \
     if (has_int) {                                                                          \
       cudaEventRecord(h->ev_fork, s);                                                       \
       cudaStreamWaitEvent(h->aux, h->ev_fork, 0);                                           \
@@ -813,15 +829,15 @@ size_t batch_stage_smem() { return t32::MB::SMEM; }
 
 // One persistent launch per RK stage over the whole work-list (MHD items of
 // 32 x 8 columns).
-static void launch_batch_stages(const BatchLaunch &B, cudaStream_t s) {
+static int launch_batch_stages(const BatchLaunch &B, cudaStream_t s) {
   const int sm = (int)MhdBuf<float, true>::smem_bytes(B.zmax);
   static_assert(QuietBuf<float, 16, true, 2, true>::bytes(0) <= t32::MB::smem_bytes(0) &&
                     QuietBuf<float, 16, true, 3, false>::bytes(0) <= t32::MB::smem_bytes(0) &&
                     QuietBuf<float, 16, false, 2, true>::bytes(0) <= t32::MB::smem_bytes(0),
                 "the quiet items' ring fits the buffer of the MHD items");
-  cudaFuncSetAttribute(k_batch_stage<F_FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  cudaFuncSetAttribute(k_batch_stage<F_MID>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  cudaFuncSetAttribute(k_batch_stage<F_LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (allow_smem(k_batch_stage<F_FIRST>) || allow_smem(k_batch_stage<F_MID>) ||
+      allow_smem(k_batch_stage<F_LAST>))
+    return SPARC_ERR_CUDA;
   const dim3 blk(t32::TX, t32::TY, 2);
   for (int st = 1; st <= 5; ++st) {
     unsigned *c = B.wctr + st;  // work counter of stage st
@@ -832,6 +848,7 @@ static void launch_batch_stages(const BatchLaunch &B, cudaStream_t s) {
     else
       k_batch_stage<F_LAST><<<B.grid, blk, (size_t)sm, s>>>(B.slots, B.items, B.counts, c, st);
   }
+  return SPARC_OK;
 }
 
 int launch_batch_step(const BatchLaunch &B, cudaStream_t s, int *nkernels) {
@@ -839,7 +856,7 @@ int launch_batch_step(const BatchLaunch &B, cudaStream_t s, int *nkernels) {
   k_batch_begin<<<(B.nslots + 255) / 256, 256, 0, s>>>(B.slots, B.nslots);
   k_batch_psr<<<B.grid, BT, B.psr_smem, s>>>(B.slots, B.pitems, B.counts, B.wctr + 0);
   k_batch_random<<<B.grid, BT, 0, s>>>(B.slots, B.nslots);
-  launch_batch_stages(B, s);
+  if (launch_batch_stages(B, s)) return SPARC_ERR_CUDA;
   k_batch_filter_xy<<<B.grid * 6, dim3(fb::TX, fb::TY), 0, s>>>(B.slots, B.xyitems, B.counts,
                                                                  B.wctr + 6);
   k_batch_filter_z<<<B.grid * 6, dim3(fb::ZX, fb::ZY, 2), filt_z_smem<float>(), s>>>(
