@@ -18,10 +18,11 @@
 namespace sparc {
 
 // D: PsrDev (FP64 sums) or Psr32 (FP32 sums); sh: the dynamic buffer, a value
-// of R and an int per pulse.  Block (32, 8); blockIdx: tile x, tile y, layer.
+// of R and an int per pulse, and no static shared memory beside it: the 48 KB that
+// a launch may take without asking hold 4096 pulses in FP64, 6144 in FP32.
+// Block (32, 8); blockIdx: tile x, tile y, layer.
 template <class R, class D>
 __device__ __forceinline__ void psr_tile(const D &P, R *sh, int maxp) {
-  __shared__ int s_n;
   const int k = P.klo + blockIdx.z;
   const int e0 = P.off[k], ne = P.off[k + 1] - e0;
   R *sT = sh;
@@ -50,10 +51,11 @@ __device__ __forceinline__ void psr_tile(const D &P, R *sh, int maxp) {
       __syncwarp();
       at += __popc(m);
     }
-    if (lane == 0) s_n = at;
+    if (lane == 0) *(int *)sh = at;  // their count, where their factors go next
   }
   __syncthreads();
-  const int kept = s_n;
+  const int kept = *(const volatile int *)sh;
+  __syncthreads();
   const long long it = *P.iter;
   const double t = (double)it * P.timestep;
   const double passes = (it == P.init) ? 2.0 : 1.0;
