@@ -16,6 +16,7 @@
 #include <cufft.h>
 
 #include <cmath>
+#include <string>
 #include <vector>
 
 #include "internal.h"
@@ -41,12 +42,38 @@ static bool fft_ok(Handle *h, cufftResult r, const char *what) {
   return false;
 }
 
+// The spectrum of `fields` velocities and the plans for them; nothing is kept
+// where one of them cannot be had.
+static int damping_plans(Handle *h, int fields) {
+  const int nx = h->nx, ny = h->ny, nz = h->nz, nh = nx / 2 + 1;
+  h->damp_fields = fields;
+  h->d_spec = (double2 *)dev_alloc(h, (size_t)fields * nh * ny * nz * sizeof(double2));
+  if (!h->d_spec) return SPARC_ERR_NOMEM;
+  // (real rows are px values apart, as in the state)
+  int n[2] = {ny, nx}, real_e[2] = {ny, h->px}, half_e[2] = {ny, nh};
+  if (fft_ok(h, cufftPlanMany(&h->fft_fwd, 2, n, real_e, 1, h->px * ny, half_e, 1, nh * ny,
+                              CUFFT_D2Z, nz * fields),
+             "cufftPlanMany (forward)")) {
+    if (fft_ok(h, cufftPlanMany(&h->fft_inv, 2, n, half_e, 1, nh * ny, real_e, 1, h->px * ny,
+                                CUFFT_Z2D, nz * fields),
+               "cufftPlanMany (inverse)")) {
+      h->fft_plans = true;
+      return SPARC_OK;
+    }
+    cufftDestroy(h->fft_fwd);
+  }
+  cudaGetLastError();  // an allocation of the library's
+  dev_free(h, h->d_spec);
+  h->d_spec = nullptr;
+  return SPARC_ERR_CUDA;
+}
+
 // The damping rates (initialize.f90:1287-1312, FP64 on the host, in the
 // reference's operation order) and the batched plans.  kay2d is the
 // horizontal wavenumber in units of 1/Rsun: kx = i (i = 0..nx/2), ky = j
 // for j <= ny/2 and ny - j above (the negative frequencies).
 int damping_setup(Handle *h) {
-  const int nx = h->nx, ny = h->ny, nz = h->nz, nh = nx / 2 + 1;
+  const int nx = h->nx, ny = h->ny, nh = nx / 2 + 1;
   const double constx = 2.0 * PI * RSUN / h->P.xlength;
   const double consty = 2.0 * PI * RSUN / h->P.ylength;
   const double kayref = 902.0;
@@ -62,32 +89,21 @@ int damping_setup(Handle *h) {
     }
   }
   h->d_damp = (double *)dev_alloc(h, rates.size() * 8);
-  // the three velocities lie one after another: one batch of 3 nz layers
-  // (2 transforms and 1 product per stage where there were 6 and 3; one field
-  // at a time where the spectrum of three does not fit)
-  h->damp_fields = 3;
-  h->d_spec = (double2 *)dev_alloc(h, (size_t)3 * nh * ny * nz * sizeof(double2));
-  if (!h->d_spec) {
-    h->damp_fields = 1;
-    h->d_spec = (double2 *)dev_alloc(h, (size_t)nh * ny * nz * sizeof(double2));
-  }
   h->d_term = (double *)dev_alloc(h, (size_t)3 * h->NP * 8);
-  if (!h->d_damp || !h->d_spec || !h->d_term) return SPARC_ERR_NOMEM;
+  if (!h->d_damp || !h->d_term) return SPARC_ERR_NOMEM;
   if (cudaMemcpyAsync(h->d_damp, rates.data(), rates.size() * 8, cudaMemcpyHostToDevice,
                       h->stream) != cudaSuccess ||
       cudaStreamSynchronize(h->stream) != cudaSuccess)
     return SPARC_ERR_CUDA;
-  // (real rows are px values apart, as in the state)
-  int n[2] = {ny, nx}, real_e[2] = {ny, h->px}, half_e[2] = {ny, nh};
-  if (!fft_ok(h, cufftPlanMany(&h->fft_fwd, 2, n, real_e, 1, h->px * ny, half_e, 1, nh * ny,
-                               CUFFT_D2Z, nz * h->damp_fields),
-              "cufftPlanMany (forward)") ||
-      !fft_ok(h, cufftPlanMany(&h->fft_inv, 2, n, half_e, 1, nh * ny, real_e, 1, h->px * ny,
-                               CUFFT_Z2D, nz * h->damp_fields),
-              "cufftPlanMany (inverse)"))
-    return SPARC_ERR_CUDA;
-  h->fft_plans = true;
-  return SPARC_OK;
+  // The three velocities lie one after another: one batch of 3 nz layers (2
+  // transforms and 1 product per stage where there were 6 and 3); one field at
+  // a time where the spectrum of three, or the library's work areas for them,
+  // cannot be had.
+  const std::string err = h->err;
+  if (!damping_plans(h, 3)) return SPARC_OK;
+  const int r = damping_plans(h, 1);
+  if (!r) h->err = err;  // nothing failed that is still wanted
+  return r;
 }
 
 // The three damping terms of the velocities of state tin (fields 1..3)
