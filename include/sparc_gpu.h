@@ -184,10 +184,14 @@ int sparc_get_zchunk(const sparc_handle *h, int *zchunk);
 
 /* Autotuner of the z extent: runs iterations first, first+1, ... of the
  * driver loop exactly as sparc_run would (they are real iterations of the
- * simulation), giving each candidate extent (16 .. 150 layers) one untimed
- * iteration and then `steps_per_trial` iterations off the filter cadence
- * timed with CUDA events; keeps the fastest.  *next receives the first
- * iteration not yet run, *best the extent chosen.  Synchronous. */
+ * simulation), giving each candidate extent (the set-up one and 12 .. 152
+ * layers; quiet equations at most 32) one untimed iteration and then
+ * `steps_per_trial` iterations off the filter cadence timed with CUDA events;
+ * keeps the fastest.  *next receives the first iteration not yet run, *best
+ * the extent chosen.  Synchronous.
+ * An MHD set-up extent below 11 (sparc_get_zchunk before any change; grids of
+ * fewer tiles than the GPU has SMs) is not a candidate, and faster than those:
+ * leave such a grid as set up, or set that extent again afterwards. */
 int sparc_tune(sparc_handle *h, int64_t first, int steps_per_trial, int64_t *next,
                int *best);
 
