@@ -167,7 +167,8 @@ void state_io_open() {
 }
 
 void state_io_close() {
-  std::lock_guard<std::mutex> use(g_use);  // no copy in flight
+  // no copy is in flight where no handle is left; otherwise the slab stays, and
+  // another handle's copy is not waited for
   std::lock_guard<std::mutex> l(g_mu);
   if (--g_handles == 0 && g_slab) {
     cudaFreeHost(g_slab);
