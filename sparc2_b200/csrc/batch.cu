@@ -84,11 +84,11 @@ int grow(Batch *b, T *&p, size_t &cap, size_t need) {
   return SPARC_OK;
 }
 
-// Rebuild the work-lists from the occupied slots and upload them with the
-// slot table (the batch stream is idle when this runs).
 // layers of a stage item at most: its depth scales sit in shared memory
 int batch_extent(int zchunk) { return std::min(std::max(11, zchunk), 1024); }
 
+// Rebuild the work-lists from the occupied slots and upload them with the
+// slot table (the batch stream is idle when this runs).
 int rebuild(Batch *b) {
   std::vector<int4> items, fitems, pitems, zitems, xyitems;
   size_t npart = 0;

@@ -83,7 +83,7 @@ struct SimT {
   // iteration bookkeeping and diagnostics (device)
   long long *iter;             // current driver iteration
   int *err;                    // device error flag (bounded waits)
-  double *partials;            // 3 per block of the last stage
+  double *partials;            // last stage: 3 per block (MHD: 2 per work item)
   double *kseg;                // MHD: KE sums of 4-layer tile segments
   unsigned int *counter;
   double *diag;                // ke, min_rho, min_p, iteration(double)
@@ -382,7 +382,6 @@ int launch_stage32(Handle *h, const SimT<float> &S, int stage, const float *a,
 int launch_psr32(Handle *h, cudaStream_t s);
 Psr32 make_psr32(Handle *h);
 int launch_batch_step(const BatchLaunch &B, cudaStream_t s, int *nkernels);
-size_t batch_stage_smem();
 int launch_filter_event32(Handle *h, bool xy, const float *in, const float *carry, float *out,
                           cudaStream_t s);
 int setup32(Handle *h);

@@ -26,11 +26,11 @@
 //     per-lane and per-row coefficients from a small table (no divergence).
 // Measured per iteration of five stages, against one shared layer tile with
 // two barriers per layer and loads at their use (before -> after): FP32
-// 256x256x300 8.74 -> 2.37 ms; FP64 64x64x128 0.308 -> 0.122 ms, 32x32x48
-// 0.300 -> 0.043 ms, 133x117x171 with a 3-D background and side CPML
-// 1.86 -> 1.07 ms.  The FP32 kernel issues 70 % of its cycles (500 thread
-// instructions per point, 200 of them addresses and copies); the FP64 one
-// 36 %, waiting on its copies.
+// 256x256x300 8.74 -> 2.34 ms; FP64 64x64x128 0.308 -> 0.121 ms, 32x32x48
+// 0.300 -> 0.044 ms, 133x117x171 with a 3-D background and side CPML
+// 1.86 -> 1.05 ms.  The FP32 kernel issues 67 % of its cycles (545 thread
+// instructions per point, half of them addresses and copies); the FP64 one
+// 50 %, at 0.57 of the measured copy rate.
 //
 // Each translation unit that includes this header defines dcoef<R>(row, m)
 // (mhd_body.cuh).

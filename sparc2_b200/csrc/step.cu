@@ -4,9 +4,10 @@
 // the FILTER_VARS passes.
 //
 // Stage kernel layout: a CTA owns a TX x TY tile of (x, y) columns and
-// marches up a chunk of z layers.  z derivatives come from an 11-deep
-// register window per z-differentiated field (the thread's own column);
-// x and y derivatives from a shared-memory layer tile with a 5-point halo.
+// marches up a chunk of z layers.  z derivatives come from an 11-deep window
+// per z-differentiated field (the thread's own column): in registers for the
+// quiet equations, in tensor memory for MHD; x and y derivatives from a
+// shared-memory layer tile with a 5-point halo.
 // Stage values are forwarded: stage k writes temp_{k+1} = a + beta_{k+1}*F_k
 // (step.f90:33) instead of F_k, so every halo and window load of the next
 // stage reads one array; stage 5 writes a + deltat*F_5 (step.f90:58).  The
@@ -81,8 +82,16 @@ __global__ void __launch_bounds__(qg::TX *Quiet64<BG1D>::TY, 2)
 // shared one's time).  At most 32 layers (256x256x300 FP32: 2.36 ms per
 // iteration at 24 and 32, 2.54 at 8; 64x64x128 FP64: 0.122 at the chosen 8,
 // 0.148 at 11 and 16, 0.133 at 4), and 8 with x/y CPML slabs, whose tiles
-// take longer than the others (133x117x171 FP64: 1.06 at 4 to 8, 1.13 at 16,
-// 1.27 at 25).
+// take longer than the others.  With slabs, ms per iteration at 4 / 8 / 16 /
+// 32 layers, 3-D background, FP64 and FP32:
+//   64x64x128    0.235 / 0.238 / 0.347 / 0.604   0.180 / 0.167 / 0.247 / 0.445
+//   96x96x150    0.466 / 0.484 / 0.571 / 0.690   0.360 / 0.410 / 0.460 / 0.724
+//   133x117x171  1.048 / 1.058 / 1.128 / 1.373   0.844 / 0.964 / 1.082 / 1.069
+//   192x160x200  1.537 / 1.471 / 1.444 / 1.620   1.143 / 1.189 / 1.204 / 1.414
+//   512x64x200   1.649 / 1.578 / 1.552 / 1.699   1.253 / 1.278 / 1.286 / 1.453
+//   256x256x300  4.455 / 4.194 / 4.138 / 4.122   3.262 / 3.170 / 3.148 / 3.233
+// so that the share of slab tiles hardly matters: wide grids give away 2 % at 8
+// and narrow ones would lose up to half at 16.
 static int quiet_zchunk(const Handle *h) {
   const int occ = h->fp32 ? 3 : 2, zmax = h->use_hpml ? 8 : QUIET_ZMAX;
   const long long tiles = (long long)((h->nx + 31) / 32) * ((h->ny + 7) / 8);
@@ -107,10 +116,11 @@ static int quiet_zchunk(const Handle *h) {
 // first, where an item costs its layers and two more (window loads, start)
 // and a layer of an edge tile one and a half of an interior one's time
 // (measured: 9,600 against 6,100 cycles in FP64, 6,100 against 4,150 in
-// FP32).  Against at most 40 layers in about seven blocks per SM: FP64
-// 40x40x48 0.505 -> 0.184 ms per iteration (4 layers), 149x151x203 4.98 ->
-// 4.78 (68), FP32 149x149x211 3.07 -> 2.95 (36), 128x160x180 1.77 -> 1.74
-// (32).
+// FP32).  ms per iteration at the chosen extent and at others (layers): FP64
+// 40x40x48 0.184 (4), 0.287 (8), 0.390 (12); 149x151x203 3.21 (52), 3.17 (24), 3.34
+// (40), 3.28 (68); 256x256x300 10.31 (76), 10.47 (40), 10.25 (80), 10.80 (100);
+// FP32 149x149x211 2.41 (36), 2.47 (24), 2.53 (40), 2.63 (72); 128x160x180
+// periodic 1.767 (32), 1.779 (20), 1.787 (40), 1.914 (48).
 static int mhd_zchunk(const Handle *h) {
   constexpr int SMS = 148, ROUNDS = 24;
   const sparc_params &P = h->P;
@@ -121,7 +131,9 @@ static int mhd_zchunk(const Handle *h) {
   mhd_interior_rect(h->nx, h->ny, np, ix0, ix1, iy0, iy1);
   const int tiles = ((h->nx + mg::TX - 1) / mg::TX) * ((h->ny + mg::TY - 1) / mg::TY);
   const int nint = ix1 > ix0 && iy1 > iy0 ? (ix1 - ix0) * (iy1 - iy0) : 0, ngen = tiles - nint;
-  // without tensor copies an interior FP64 layer costs as much as an edge one
+  // without tensor copies an interior FP64 layer costs nearly as much as an edge
+  // one (odd rows, which are left unpadded only where padding would pass the
+  // 32-bit indexing)
   const double ratio = !h->fp32 && (h->px & 1) ? 1.15 : 1.5;
   int best = std::min(h->nz, 40), last = 0;
   double least = 1e300;

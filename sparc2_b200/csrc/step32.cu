@@ -825,8 +825,6 @@ __global__ void __launch_bounds__(BT)
   }
 }
 
-size_t batch_stage_smem() { return t32::MB::SMEM; }
-
 // One persistent launch per RK stage over the whole work-list (MHD items of
 // 32 x 8 columns).
 static int launch_batch_stages(const BatchLaunch &B, cudaStream_t s) {
