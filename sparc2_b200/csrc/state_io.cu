@@ -270,6 +270,9 @@ __global__ void k_narrow(const double *__restrict__ in, long long n, float *__re
     if (!cuda_ok(h, (x), "state conversion")) return SPARC_ERR_CUDA; \
   } while (0)
 
+// (A face's CPML fields fit in a free buffer, half the state in FP64: a slab is
+// no thicker than the boundary block, 12 of 23 points at most, so its 6 (quiet: 2)
+// fields are below 3.2 (1.1) state fields, and a buffer holds 4 (2.5).)
 // stored = float(sc * a), carry 0
 int set_state32(Handle *h, const double *a, const double *psi) {
   const long long VN = (long long)h->V * h->N, half = VN / 2;
